@@ -498,6 +498,13 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
         }
       }
     }
+    // The next bias tile is written by TMA, through the async proxy: the arrival alone orders this thread's reads only
+    // against other generic accesses, and a read still in flight could return the next step's bias (one row in some
+    // hundred million was, before the fence).
+    auto release_bias = [&]() {
+      ptx::fence_proxy_async();
+      ptx::mbar_arrive(ptx::smem_u32(&bars->bias_free));
+    };
     for_each_step<kDKV>(p, s, tile0, head, [&](int, int srow0, int qh) {
       w.wait(ptx::smem_u32(&bars->t_full), cnt & 1u);
       ptx::tc_fence_after();
@@ -527,7 +534,7 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
             asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                          : "=r"(bcol[4 * q4]), "=r"(bcol[4 * q4 + 1]), "=r"(bcol[4 * q4 + 2]), "=r"(bcol[4 * q4 + 3])
                          : "r"(rowbase + (((c16 + q4) ^ (row & 7)) << 4)));
-          if (ch == 1) ptx::mbar_arrive(ptx::smem_u32(&bars->bias_free));   // this thread has read its row
+          if (ch == 1) release_bias();   // this thread has read its row
         } else if (staged) {
           if (ch == 0) {
             w.wait(ptx::smem_u32(&bars->bias_full), cnt & 1u);
@@ -543,7 +550,7 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
             asm volatile("ld.shared.u16 %0, [%1];" : "=r"(hi) : "r"(box + q1l * 128 + ((kchunk ^ (q1l & 7)) << 4)));
             bcol[e] = lo | (hi << 16);
           }
-          if (ch == 1) ptx::mbar_arrive(ptx::smem_u32(&bars->bias_free));   // this thread has read its column
+          if (ch == 1) release_bias();   // this thread has read its column
         } else if (kDKV && p.bias) {
           const int kk = mine < p.maxk ? mine : p.maxk - 1;
           const unsigned short* bsrc = static_cast<const unsigned short*>(p.bias) + bias_bh + kk;
