@@ -190,7 +190,7 @@ int hstu_jagged_fwd_kernel_kind(const HstuJaggedArgs* args) {
   int rc = validate(args);
   if (rc) return rc;
   const hstu::KParams p = to_params(args, nullptr, 0);
-  return wants_tc(args, p) ? 1 : 0;
+  return wants_tc(args, p) && args->dim_qk == args->dim_v && args->dim_qk % 64 == 0 ? 1 : 0;
 }
 
 // `paged` (hstu_paged only): parameters that carry the page table, for the pre-pass's consistency check.

@@ -1,5 +1,6 @@
-// HSTU jagged backward on Blackwell tensor cores (tcgen05 + TMEM + TMA), bf16 / fp16, Dqk = Dv in {64, 128},
-// mask tril / none, the reference's order x = alpha (S + bias).  Everything else runs on hstu_bwd_generic.cu.
+// HSTU jagged backward on Blackwell tensor cores (tcgen05 + TMEM + TMA), bf16 / fp16, head dims up to 128 (multiples of
+// 8 for Dqk, of 16 for Dv; D = 64 or 128 is the tile width that holds both, TMA reads zeros past a row's end), mask tril /
+// none, the reference's order x = alpha (S + bias).  Everything else runs on hstu_bwd_generic.cu.
 //
 // One kernel template, launched twice with one persistent CTA per SM (the tiles of a pass come from a list the
 // pre-pass wrote - only tiles that exist - through a counter in the workspace; the producer thread draws them and
@@ -182,6 +183,9 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
   constexpr uint32_t kColT1b = kDKV ? kColT1 : (D == 128 ? 256u : 384u);
   const KParams& p = bp.f;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // 64-wide halves of the tiles of width Dqk (A1, B1) and Dv (A2, B2); what a tile has not is neither loaded nor read
+  const int halves1 = kHalves == 1 ? 1 : (p.dqk + 63) >> 6;
+  const int halves2 = kHalves == 1 ? 1 : (p.dv + 63) >> 6;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -295,11 +299,11 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
         if (tiles_done > 0) w.wait(ptx::smem_u32(&bars->acc_full), (tiles_done - 1u) & 1u);
         if (*reinterpret_cast<volatile int*>(&bars->abort_flag)) break;
         const uint32_t afull = ptx::smem_u32(&bars->a_full);
-        ptx::mbar_expect_tx(afull, 2 * kTileBytes);
+        ptx::mbar_expect_tx(afull, (halves1 + halves2) * kHalfBytes);
 #pragma unroll
         for (int hf = 0; hf < kHalves; ++hf) {
-          ptx::tma_load_3d(sm_a + hf * kHalfBytes, &tm_a1, afull, hf * 64, a_head, static_cast<int>(a_row));
-          ptx::tma_load_3d(sm_a + kTileBytes + hf * kHalfBytes, &tm_a2, afull, hf * 64, a_head, static_cast<int>(a_row));
+          if (hf < halves1) ptx::tma_load_3d(sm_a + hf * kHalfBytes, &tm_a1, afull, hf * 64, a_head, static_cast<int>(a_row));
+          if (hf < halves2) ptx::tma_load_3d(sm_a + kTileBytes + hf * kHalfBytes, &tm_a2, afull, hf * 64, a_head, static_cast<int>(a_row));
         }
         for_each_step<kDKV>(p, s, tile0, head, [&](int sh, int srow0, int qh) {
           const uint32_t stage = cnt & 1u;
@@ -317,12 +321,12 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
               ptx::tma_load_2d(sm_bias + hf * (kTileM * 128), &tm_bias, bfull, bcol0 + hf * 64, brow);
           }
           w.wait(ptx::smem_u32(&bars->b_free[stage]), ((cnt >> 1) & 1u) ^ 1u);
-          ptx::mbar_expect_tx(full, 2 * kTileBytes);
+          ptx::mbar_expect_tx(full, (halves1 + halves2) * kHalfBytes);
           const int row = static_cast<int>(b_row0) + srow0;
 #pragma unroll
           for (int hf = 0; hf < kHalves; ++hf) {
-            ptx::tma_load_3d(sm_b + stage * 2 * kTileBytes + hf * kHalfBytes, &tm_b1, full, hf * 64, sh, row);
-            ptx::tma_load_3d(sm_b + stage * 2 * kTileBytes + kTileBytes + hf * kHalfBytes, &tm_b2, full, hf * 64, sh, row);
+            if (hf < halves1) ptx::tma_load_3d(sm_b + stage * 2 * kTileBytes + hf * kHalfBytes, &tm_b1, full, hf * 64, sh, row);
+            if (hf < halves2) ptx::tma_load_3d(sm_b + stage * 2 * kTileBytes + kTileBytes + hf * kHalfBytes, &tm_b2, full, hf * 64, sh, row);
           }
           ++cnt;
         });
@@ -391,7 +395,9 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
     // (an elected thread, not `lane == 0`: the compiler then keeps descriptors and barrier addresses in uniform registers)
     if (ptx::elect_one()) {
       constexpr uint32_t idesc_t = ptx::umma_idesc_f16(BPack<T>::kFormat, kTileM, kTileN, 0);
-      constexpr uint32_t idesc_acc = ptx::umma_idesc_f16(BPack<T>::kFormat, kTileM, D, 1);
+      const uint32_t idesc_acc1 = ptx::umma_idesc_f16(BPack<T>::kFormat, kTileM, p.dv, 1);
+      const uint32_t idesc_acc2 = ptx::umma_idesc_f16(BPack<T>::kFormat, kTileM, (p.dqk + 15) & ~15, 1);
+      const bool half1 = p.dqk <= D / 2, half2 = p.dv <= D / 2;   // the upper half of the contraction holds only zeros
       constexpr uint64_t kDescK = ptx::umma_desc_sw128_hi(16, 1024);           // K-major tiles
       constexpr uint64_t kDescN = ptx::umma_desc_sw128_hi(kHalfBytes, 1024);   // the same tiles read N-major
       const uint64_t a1 = kDescK | static_cast<uint64_t>(sm_a >> 4);
@@ -409,8 +415,8 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
         auto part = [&](int ks, uint32_t acc) {
           const uint32_t ucol = (ks >> 2) * 64 + (ks & 3) * 8;
           const uint64_t off = static_cast<uint64_t>((ks * 2048) >> 4);
-          if (kDKV) ptx::mma_ts(tmem + kColAcc1, tmem + kColT1 + ucol, b2n + off, idesc_acc, acc);
-          ptx::mma_ts(tmem + kColAcc2, tmem + col_u2 + ucol, b1n + off, idesc_acc, acc);
+          if (kDKV) ptx::mma_ts(tmem + kColAcc1, tmem + kColT1 + ucol, b2n + off, idesc_acc1, acc);
+          ptx::mma_ts(tmem + kColAcc2, tmem + col_u2 + ucol, b1n + off, idesc_acc2, acc);
         };
         w.wait(ptx::smem_u32(&bars->u_full[0]), c & 1u);
         ptx::tc_fence_after();
@@ -438,17 +444,21 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
         const uint64_t b1 = kDescK | static_cast<uint64_t>((sm_b + stage * 2 * kTileBytes) >> 4);
         const uint64_t b2 = kDescK | static_cast<uint64_t>((sm_b + stage * 2 * kTileBytes + kTileBytes) >> 4);
         const uint32_t col_t1 = (cnt & 1u) ? kColT1b : kColT1;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          const uint64_t off = static_cast<uint64_t>(((ks >> 2) * kHalfBytes + (ks & 3) * 32) >> 4);
-          ptx::mma_ss(tmem + col_t1, a1 + off, b1 + off, idesc_t, ks > 0 ? 1u : 0u);
-        }
-        auto t2_product = [&]() {
-#pragma unroll
-          for (int ks = 0; ks < D / 16; ++ks) {
+        auto product = [&](uint32_t col, uint64_t a, uint64_t b, bool half) {
+          auto one = [&](int ks) {
             const uint64_t off = static_cast<uint64_t>(((ks >> 2) * kHalfBytes + (ks & 3) * 32) >> 4);
-            ptx::mma_ss(tmem + kColT2, a2 + off, b2 + off, idesc_t, ks > 0 ? 1u : 0u);
+            ptx::mma_ss(col, a + off, b + off, idesc_t, ks > 0 ? 1u : 0u);
+          };
+#pragma unroll
+          for (int ks = 0; ks < D / 32; ++ks) one(ks);
+          if (!half) {
+#pragma unroll
+            for (int ks = D / 32; ks < D / 16; ++ks) one(ks);
           }
+        };
+        product(tmem + col_t1, a1, b1, half1);
+        auto t2_product = [&]() {
+          product(tmem + kColT2, a2, b2, half2);
           ptx::mma_commit(ptx::smem_u32(&bars->t_full));
         };
         // dQ pass: first half of the last step's accumulate products, this step's dP product, then the second half
@@ -670,12 +680,14 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
     }
     const int col0 = grp * (D / 2);
     const long long tok = (kDKV ? s.k0 : s.q0) + mine;
-    T* out2 = static_cast<T*>(kDKV ? bp.dk : bp.dq) + (tok * heads + head) * D + col0;
-    T* out1 = kDKV ? static_cast<T*>(bp.dv) + (tok * heads + head) * D + col0 : nullptr;
+    T* out2 = static_cast<T*>(kDKV ? bp.dk : bp.dq) + (tok * heads + head) * p.dqk + col0;
+    T* out1 = kDKV ? static_cast<T*>(bp.dv) + (tok * heads + head) * p.dv + col0 : nullptr;
 #pragma unroll 1
     for (int ch = 0; ch < D / 64; ++ch) {
 #pragma unroll 1
       for (int which = kDKV ? 0 : 1; which < 2; ++which) {
+        const int room = (which == 0 ? p.dv : p.dqk) - col0 - ch * 32;   // columns of the row from here on
+        if (room <= 0) continue;
         uint32_t acc[32];
         if (cnt > first) {
           ptx::tmem_ld32(tmem + lane_base + (which == 0 ? kColAcc1 : kColAcc2) + col0 + ch * 32, acc);
@@ -693,7 +705,7 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
             u.y = BPack<T>::pack(__uint_as_float(acc[q4 * 8 + 2]), __uint_as_float(acc[q4 * 8 + 3]));
             u.z = BPack<T>::pack(__uint_as_float(acc[q4 * 8 + 4]), __uint_as_float(acc[q4 * 8 + 5]));
             u.w = BPack<T>::pack(__uint_as_float(acc[q4 * 8 + 6]), __uint_as_float(acc[q4 * 8 + 7]));
-            dst[q4] = u;
+            if (q4 * 8 < room) dst[q4] = u;
           }
         }
       }
@@ -777,7 +789,8 @@ cudaError_t launch_bwd_tc_t(const BwdParams& bp, int dtype, int num_sms, cudaStr
 bool bwd_tc_supported(const BwdParams& bp, int dtype) {
   const KParams& p = bp.f;
   if (dtype != HSTU_DTYPE_BF16 && dtype != HSTU_DTYPE_FP16) return false;
-  if (p.dqk != p.dv || (p.dqk != 64 && p.dqk != 128)) return false;
+  // (the same rule, for the same reasons, as the forward's)
+  if (p.dqk > 128 || p.dv > 128 || p.dqk % 8 != 0 || p.dv % 16 != 0) return false;
   if (p.mask_type != HSTU_MASK_TRIL && p.mask_type != HSTU_MASK_NONE) return false;
   if (p.flags & (HSTU_FLAG_ALPHA_BEFORE_BIAS | HSTU_FLAG_FORCE_GENERIC)) return false;
   if (p.total_q > 0x7fffff00ll || p.total_k > 0x7fffff00ll) return false;
@@ -791,10 +804,11 @@ bool bwd_tc_supported(const BwdParams& bp, int dtype) {
 // Returns cudaSuccess, a CUDA error, or cudaErrorNotSupported when the tensor maps could not be encoded.
 cudaError_t launch_bwd_tc(const BwdParams& bp, int dtype, int num_sms, cudaStream_t stream) {
   const KParams& p = bp.f;
+  const bool wide = p.dqk > 64 || p.dv > 64;
   if (dtype == HSTU_DTYPE_BF16)
-    return p.dqk == 128 ? launch_bwd_tc_t<128, __nv_bfloat16>(bp, dtype, num_sms, stream)
+    return wide ? launch_bwd_tc_t<128, __nv_bfloat16>(bp, dtype, num_sms, stream)
                         : launch_bwd_tc_t<64, __nv_bfloat16>(bp, dtype, num_sms, stream);
-  return p.dqk == 128 ? launch_bwd_tc_t<128, __half>(bp, dtype, num_sms, stream) : launch_bwd_tc_t<64, __half>(bp, dtype, num_sms, stream);
+  return wide ? launch_bwd_tc_t<128, __half>(bp, dtype, num_sms, stream) : launch_bwd_tc_t<64, __half>(bp, dtype, num_sms, stream);
 }
 
 }  // namespace hstu

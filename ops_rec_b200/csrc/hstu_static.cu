@@ -58,6 +58,15 @@ HSTU_API int hstu_jagged_fwd_static(const HstuJaggedArgs* args, void* stream) {
   uint64_t need = 0;
   int rc = hstu_jagged_fwd_get_workspace_size(args, &need);  // validates args; host arithmetic only
   if (rc) return rc;
+  // (head dims that are not a tile width of the tensor-core kernel: the generic kernel needs no list, so it takes the
+  // batches whose list is too long)
+  HstuJaggedArgs listless = *args;
+  if (need > HSTU_STATIC_SCRATCH_BYTES && hstu_jagged_fwd_kernel_kind(args) == 0) {
+    listless.flags |= HSTU_FLAG_FORCE_GENERIC;
+    args = &listless;
+    rc = hstu_jagged_fwd_get_workspace_size(args, &need);
+    if (rc) return rc;
+  }
   if (need > HSTU_STATIC_SCRATCH_BYTES)
     return hstu_set_last_error(HSTU_E_SCRATCH_LIMIT, "hstu_jagged_fwd_static: the work list of this call does not "
                                                      "fit the built-in scratch block; use hstu_jagged_fwd with a "

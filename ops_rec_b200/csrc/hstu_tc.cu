@@ -1,4 +1,8 @@
-// HSTU jagged attention forward on the sm_100a tensor cores (tcgen05 + TMEM), bf16 / fp16, head dim 64 or 128.
+// HSTU jagged attention forward on the sm_100a tensor cores (tcgen05 + TMEM), bf16 / fp16, head dims up to 128.
+//
+// D = 64 or 128 is the tile width the kernel is built for; a call's Dqk and Dv are any multiples of 8 / 16 up to it and
+// need not agree.  TMA fills what a 64-wide box reads past a row's end with zeros and clips what it writes there, so the
+// tiles need no padding in memory; a 64-wide half that a dim does not reach is neither loaded nor multiplied.
 //
 // One persistent CTA per SM walks the scheduler's work list.  A work item is a (sequence, head, 256-row q-pair):
 // two 128-row Q tiles that share every K/V tile fetched.  Per K tile and Q tile:
@@ -400,6 +404,9 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Waiter w{&bars->abort_flag, p.ws_header};
+  // 64-wide halves that Q / K and V have (constant for D = 64)
+  const int halves_qk = C::kHalves == 1 ? 1 : (p.dqk + 63) >> 6;
+  const int halves_v = C::kHalves == 1 ? 1 : (p.dv + 63) >> 6;
 
   if (threadIdx.x == 0) {
     ptx::prefetch_tensormap(&tm_q);
@@ -464,11 +471,11 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
           const uint32_t full = ptx::smem_u32(&bars->q_full[t]);
           w.wait(ptx::smem_u32(&bars->q_free[t]), (q_uses[t] & 1u) ^ 1u);
           if (w.aborted()) return;  // a wait gave up somewhere: request nothing more, touch no barrier
-          ptx::mbar_expect_tx(full, C::kTileBytes);
+          ptx::mbar_expect_tx(full, halves_qk * C::kHalfBytes);
           const int row = static_cast<int>(it.s.q0) + it.r0 + t * kTileM;
 #pragma unroll
           for (int hf = 0; hf < C::kHalves; ++hf)
-            ptx::tma_load_3d(sm_q + t * C::kTileBytes + hf * C::kHalfBytes, &tm_q, full, hf * 64, it.h, row);
+            if (hf < halves_qk) ptx::tma_load_3d(sm_q + t * C::kTileBytes + hf * C::kHalfBytes, &tm_q, full, hf * 64, it.h, row);
           ++q_uses[t];
         };
         // Order: Q tile 0, K tile 0, Q tile 1, V tile 0, ...  Tile 1's buffer is released last by the previous
@@ -491,12 +498,13 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
             const uint32_t full = ptx::smem_u32(&bars->kv_full[stage]);
             w.wait(ptx::smem_u32(&bars->kv_free[stage]), (use & 1u) ^ 1u);
             if (w.aborted()) break;
-            ptx::mbar_expect_tx(full, C::kTileBytes);
+            const int halves = kv == 0 ? halves_qk : halves_v;
+            ptx::mbar_expect_tx(full, halves * C::kHalfBytes);
             const CUtensorMap* tm = from_cache ? &tm_cache : (kv == 0 ? &tm_k : &tm_v);
             const int trow = from_cache ? static_cast<int>((pid * 2 + kv) * kTileN) : row;
 #pragma unroll
             for (int hf = 0; hf < C::kHalves; ++hf)
-              ptx::tma_load_3d(sm_ring + stage * C::kTileBytes + hf * C::kHalfBytes, tm, full, hf * 64, it.hk, trow);
+              if (hf < halves) ptx::tma_load_3d(sm_ring + stage * C::kTileBytes + hf * C::kHalfBytes, tm, full, hf * 64, it.hk, trow);
             ++ring_pos;
             if (j == 0 && kv == 0) load_q(1);
           }
@@ -528,7 +536,8 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
     if (ptx::elect_one()) {
       const int t = warp == 1 ? 0 : 1;
       constexpr uint32_t idesc_qk = ptx::umma_idesc_f16(Pack<T>::kFormat, kTileM, kTileN, 0);
-      constexpr uint32_t idesc_pv = ptx::umma_idesc_f16(Pack<T>::kFormat, kTileM, D, 1);
+      const uint32_t idesc_pv = ptx::umma_idesc_f16(Pack<T>::kFormat, kTileM, p.dv, 1);
+      const bool half_k = p.dqk <= D / 2;   // the upper half of the contraction holds nothing but zeros
       // descriptor templates (everything but the start address): K-major Q / K tiles, N-major V tiles
       constexpr uint64_t kDescK = ptx::umma_desc_sw128_hi(16, 1024);
       constexpr uint64_t kDescV = ptx::umma_desc_sw128_hi(C::kHalfBytes, 1024);
@@ -612,10 +621,15 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
           if (do_qk) {
             // S_t = Q_t . K(step)^T
             const uint64_t kbase = kDescK | static_cast<uint64_t>((sm_ring + st_k * C::kTileBytes) >> 4);
-#pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
+            auto qk = [&](int ks) {
               const uint64_t off = static_cast<uint64_t>(((ks >> 2) * C::kHalfBytes + (ks & 3) * 32) >> 4);
               ptx::mma_ss(col_s, qbase + off, kbase + off, idesc_qk, ks > 0 ? 1u : 0u);
+            };
+#pragma unroll
+            for (int ks = 0; ks < D / 32; ++ks) qk(ks);
+            if (!half_k) {
+#pragma unroll
+              for (int ks = D / 32; ks < D / 16; ++ks) qk(ks);
             }
             if (kBias == 2) {
               // S_t += bias tile, 16 columns per product; only the slices that lie wholly inside the sequence
@@ -823,7 +837,7 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
       if (tile_r0 >= ot.lq) return;
       const int col0 = grp * (D / 2);
       const bool row_ok_t = tile_r0 + row < ot.lq;
-      T* orow = static_cast<T*>(p.out) + ((ot.q0 + tile_r0 + row) * p.hq + ot.h) * D + col0;
+      T* orow = static_cast<T*>(p.out) + ((ot.q0 + tile_r0 + row) * p.hq + ot.h) * p.dv + col0;
       if (ot.n > 0) {
         const uint32_t t_o = tmem + lane_base + (t == 0 ? kColO0 : C::kColO1) + col0;
         w.wait(ptx::smem_u32(&bars->o_full[t]), (t == 0 ? o_uses0 : o_uses1) & 1u);
@@ -834,6 +848,7 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
         const bool by_tma = C::kOutBytes > 0 && tile_r0 + kTileM <= ot.lq;
 #pragma unroll 1
         for (int ch = 0; ch < D / 64; ++ch) {
+          if (col0 + ch * 32 >= p.dv) break;   // (the stores clip what is left: TMA at the tensor's edge, 16 bytes at a time below)
           uint32_t orr[32];
           ptx::tmem_ld32(t_o + ch * 32, orr);
           ptx::tmem_wait_ld();
@@ -873,7 +888,7 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
               u.y = Pack<T>::pack(__uint_as_float(orr[q4 * 8 + 2]), __uint_as_float(orr[q4 * 8 + 3]));
               u.z = Pack<T>::pack(__uint_as_float(orr[q4 * 8 + 4]), __uint_as_float(orr[q4 * 8 + 5]));
               u.w = Pack<T>::pack(__uint_as_float(orr[q4 * 8 + 6]), __uint_as_float(orr[q4 * 8 + 7]));
-              dst[q4] = u;
+              if (col0 + ch * 32 + q4 * 8 < p.dv) dst[q4] = u;
             }
           }
         }
@@ -882,7 +897,8 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
       } else if (row_ok_t) {
         uint4* dst = reinterpret_cast<uint4*>(orow);
 #pragma unroll
-        for (int q4 = 0; q4 < D / 16; ++q4) dst[q4] = make_uint4(0, 0, 0, 0);
+        for (int q4 = 0; q4 < D / 16; ++q4)
+          if (col0 + q4 * 8 < p.dv) dst[q4] = make_uint4(0, 0, 0, 0);
       }
     };
     // the S tiles arrive in the order the MMA issuers alternate: tile 0 step j, tile 1 step j, tile 0 step j+1 ..
@@ -1148,7 +1164,10 @@ bool make_tile_map(CUtensorMap* m, const void* base, long long tokens, int heads
 
 bool tc_supported(const KParams& p, int dtype) {
   if (dtype != HSTU_DTYPE_BF16 && dtype != HSTU_DTYPE_FP16) return false;
-  if (p.dqk != p.dv || (p.dqk != 64 && p.dqk != 128)) return false;
+  // multiples of 8: TMA wants 16-byte strides; of 16 for dv: the N of P.V.  Beyond 128 the accumulators do not fit the
+  // tensor memory.  (Forward and backward of 24 sequences of 100 - 600 rows, 4 heads, dims 64 / 128: 4807 us on the
+  // CUDA-core kernels, 177 us here.)
+  if (p.dqk > 128 || p.dv > 128 || p.dqk % 8 != 0 || p.dv % 16 != 0) return false;
   // a custom mask takes the operand slot of the bias (plain loads), so the two together run on the generic kernel
   if (p.mask_type == HSTU_MASK_CUSTOM && (!p.mask || p.bias)) return false;
   if (p.hq > 0xffff || p.total_q > 0x7fffff00ll || p.total_k > 0x7fffff00ll) return false;
@@ -1201,11 +1220,12 @@ cudaError_t launch_tc(const KParams& p_in, int dtype, int num_sms, cudaStream_t 
          : bias_mode == 2 ? launch_inst<DD, TT, 2, false>(p, mq, mk, mv, mb, mo, mc, vec_ok, g, stream)             \
          : bias_mode == 1 ? launch_inst<DD, TT, 1, false>(p, mq, mk, mv, mb, mo, mc, vec_ok, g, stream)             \
                           : launch_inst<DD, TT, 0, false>(p, mq, mk, mv, mb, mo, mc, vec_ok, g, stream)
+  const bool wide = p.dqk > 64 || p.dv > 64;
   if (dtype == HSTU_DTYPE_BF16) {
-    if (p.dqk == 128) { HSTU_TC_CASE(128, __nv_bfloat16); }
+    if (wide) { HSTU_TC_CASE(128, __nv_bfloat16); }
     HSTU_TC_CASE(64, __nv_bfloat16);
   }
-  if (p.dqk == 128) { HSTU_TC_CASE(128, __half); }
+  if (wide) { HSTU_TC_CASE(128, __half); }
   HSTU_TC_CASE(64, __half);
 #undef HSTU_TC_CASE
 }

@@ -398,3 +398,13 @@ def test_staged_bias_tiles_are_read_before_they_are_replaced():
         res = cabi.hstu_jagged_backward(grad, q, k, v, None, bias, 0, 1024, 1024, 0.0, off, off, ctx, tgt, 1, 1.0 / 128)
         first = first or res
         assert all(torch.equal(x, y) for x, y in zip(first, res))
+
+
+@pytest.mark.parametrize("Dqk,Dv", [(8, 16), (32, 32), (64, 128), (72, 80), (96, 64), (128, 32)])
+@pytest.mark.parametrize("dtype,bias,tgt", [(BF16, False, 5), (FP16, True, 0)])
+def test_head_dims_narrower_than_a_tile(Dqk, Dv, dtype, bias, tgt):
+    grad, args = make_bwd_case(4, 4, 2, Dqk, Dv, 270, dtype, seed=Dqk + Dv, bias=bias, tgt=tgt, g=1 if tgt else 0,
+                               alpha=1.0 / Dqk)
+    got, status = run_bwd(grad, args)
+    assert status == 0
+    assert_bwd_parity(got, grad, args, label=f"{Dqk}x{Dv} {dtype}")

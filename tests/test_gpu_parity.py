@@ -375,3 +375,14 @@ def test_custom_mask_with_bias_takes_the_generic_kernel():
     out, st = run_cabi(args)
     assert st == 0
     assert_parity(out, args, label="mask + bias")
+
+
+@pytest.mark.parametrize("Dqk,Dv", [(8, 16), (32, 32), (48, 16), (64, 128), (72, 80), (96, 64), (120, 112), (128, 32)])
+@pytest.mark.parametrize("dtype,rab,tgt", [(BF16, None, 5), (FP16, "batch", 0), (BF16, "shared3", 9)])
+def test_head_dims_narrower_than_a_tile(Dqk, Dv, dtype, rab, tgt):
+    """Dqk and Dv any multiples of 8 / 16 up to 128 run on the tensor-core kernel, in tiles of 64 or 128; sequence lengths
+    around the 128-row tiles (whole tiles leave by TMA stores, cut ones row by row)."""
+    args = make_case(6, 4, 2, Dqk, Dv, 120, 270, dtype, seed=Dqk + Dv, rab=rab, tgt=tgt, g=1 if tgt else 0)
+    out, status = run_cabi(args)
+    assert status == 0
+    assert_parity(out, args, label=f"{Dqk}x{Dv} {dtype} {rab}")
