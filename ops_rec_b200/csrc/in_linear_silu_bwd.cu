@@ -9,13 +9,11 @@
 //     bias_grad = column sums of dL (fp32);  dL is then rounded to the element type
 //     x_grad = dL . weight  [m, k];   weight_grad = dL^T . x  [n, k]            fp32 accumulation, one rounding
 //
-// Three HBM-bound passes and two tensor-core products:
-//   silu_grad_kernel   one read of g and linear_output -> dL [m, n] and its transpose dLT [n, m'] (through a shared-
-//                      memory tile, so both are written with 16-byte stores) + per-row-block column sums of dL
-//   transpose16_kernel weight -> weight^T [k, n], x -> x^T [k, m']  (m' = m rounded up to 8: TMA wants 16-byte pitches)
+//   silu_grad_kernel   one read of g and linear_output -> dL [m, n] + per-row-block column sums of dL; HBM-bound
 //   colsum_kernel      the row-block sums -> bias_grad, in a fixed order (bitwise reproducible; no atomics)
-//   launch_gemm_abt    x_grad = dL . (weight^T)^T and weight_grad = dLT . (x^T)^T on the forward's tcgen05 pipeline
-//                      (both operands K-major, which is why the transposes are materialised)
+//   launch_product     x_grad = dL . weight and weight_grad = dL^T . x on the forward's tcgen05 pipeline, which reads
+//                      dL, weight and x as they lie.  (Forward + backward of 65536 rows of width 1024: 2448 us with transposed
+//                      copies of all three and one-CTA tiles, 1863 us)
 // All intermediates live in the caller's workspace.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -24,13 +22,15 @@
 
 namespace hstu {
 
-cudaError_t launch_gemm_abt(const void* a, long long rows_a, long long lda, const void* b, int rows_b, long long ldb,
-                            long long kdim, void* out, int dtype, uint32_t* status, cudaStream_t stream);
+uint64_t product_partial_bytes(long long m, int n, long long k);
+cudaError_t launch_product(const void* a, bool trans_a, const void* b, long long m, int n, long long k, void* out,
+                           float* partial, int dtype, uint32_t* status, cudaStream_t stream);
 
 namespace {
 
-constexpr int kBt = 64;          // tile edge of the element-wise and transpose passes
 constexpr int kBtThreads = 256;
+constexpr int kBtCols = 256;     // columns of an element-wise CTA: 32 lanes x 8
+constexpr int kSumGroups = 8;    // row-block groups a column sum is added up in
 
 template <typename T> struct Cvt;
 template <> struct Cvt<__nv_bfloat16> {
@@ -55,121 +55,114 @@ struct SiluGradParams {
   int width[4], start[5];  // column range of each in the concatenated [m, n]
   const void* lo;          // linear_output [m, n]
   void* dl;                // [m, n]
-  void* dlt;               // [n, ldm]
-  float* partial;          // [ceil(m / 64), n] column sums per row block
-  long long m, ldm;
-  int n;
+  float* partial;          // [ceil(m / rows), n] column sums per row block
+  long long m;
+  int n, rows;             // rows: rows per CTA, a multiple of 32
 };
 
-// One 64 x 64 tile of [m, n] per CTA; a thread owns two 8-column pieces (one row each) of it.
+// sigmoid(x) from one ex2 and one reciprocal (each within 2 ulp; the result feeds a 16-bit rounding or a column sum)
+__device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+
+// p.rows x 256 columns of [m, n] per CTA: a thread owns 8 columns and every eighth row of the block, four rows' loads in
+// flight.  (An IEEE division per element made this pass issue-bound: two SFU operations and about ten others are left.)
 template <typename T>
 __global__ void __launch_bounds__(kBtThreads) silu_grad_kernel(const SiluGradParams p) {
-  __shared__ unsigned short s_t[kBt][kBt + 8];   // the tile of dL in the element type, for the transposed store
-  const int tid = threadIdx.x;
-  const int c0 = blockIdx.x * kBt;
-  const long long r0 = static_cast<long long>(blockIdx.y) * kBt;
-  const int piece = tid & 7;                     // columns c0 + 8 piece ..
-  const int col = c0 + piece * 8;
+  __shared__ float s_part[kBtThreads / 32][kBtCols];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int col = blockIdx.x * kBtCols + lane * 8;
+  const long long r0 = static_cast<long long>(blockIdx.y) * p.rows;
+  const long long r1 = r0 + p.rows < p.m ? r0 + p.rows : p.m;
   float csum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (col < p.n) {
+    const int which = (col >= p.start[1]) + (col >= p.start[2]) + (col >= p.start[3]);
+    const int w = which == 0 ? p.width[0] : which == 1 ? p.width[1] : which == 2 ? p.width[2] : p.width[3];
+    const int st = which == 0 ? p.start[0] : which == 1 ? p.start[1] : which == 2 ? p.start[2] : p.start[3];
+    const T* g = static_cast<const T*>(which == 0 ? p.grad[0] : which == 1 ? p.grad[1] : which == 2 ? p.grad[2] : p.grad[3]) +
+                 (col - st);
+    const T* lo = static_cast<const T*>(p.lo) + col;
+    T* dl = static_cast<T*>(p.dl) + col;
+    for (long long row = r0 + warp; row < r1; row += 32) {
+      uint4 gv[4], lv[4];
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int lr = (tid >> 3) + half * 32;       // row inside the tile
-    const long long row = r0 + lr;
-    uint4 out = make_uint4(0, 0, 0, 0);
-    if (row < p.m && col < p.n) {
-      const int which = (col >= p.start[1]) + (col >= p.start[2]) + (col >= p.start[3]);
-      const T* g = static_cast<const T*>(which == 0 ? p.grad[0] : which == 1 ? p.grad[1] : which == 2 ? p.grad[2] : p.grad[3]);
-      const int w = which == 0 ? p.width[0] : which == 1 ? p.width[1] : which == 2 ? p.width[2] : p.width[3];
-      const int st = which == 0 ? p.start[0] : which == 1 ? p.start[1] : which == 2 ? p.start[2] : p.start[3];
-      const uint4 gv = *reinterpret_cast<const uint4*>(g + row * w + (col - st));
-      const uint4 lv = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.lo) + row * p.n + col);
-      const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, lw[4] = {lv.x, lv.y, lv.z, lv.w};
-      uint32_t ow[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 g2 = Cvt<T>::up(gw[e]), l2 = Cvt<T>::up(lw[e]);
-        const float s0 = 1.f / (1.f + __expf(-l2.x)), s1 = 1.f / (1.f + __expf(-l2.y));
-        const float d0 = g2.x * (s0 * (1.f + l2.x * (1.f - s0))), d1 = g2.y * (s1 * (1.f + l2.y * (1.f - s1)));
-        csum[2 * e] += d0;
-        csum[2 * e + 1] += d1;
-        ow[e] = Cvt<T>::down(d0, d1);
+      for (int i = 0; i < 4; ++i) {
+        const long long r = row + 8 * i;
+        if (r < r1) {
+          gv[i] = __ldcs(reinterpret_cast<const uint4*>(g + r * w));
+          lv[i] = __ldcs(reinterpret_cast<const uint4*>(lo + r * p.n));
+        }
       }
-      out = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-      *reinterpret_cast<uint4*>(static_cast<T*>(p.dl) + row * p.n + col) = out;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const long long r = row + 8 * i;
+        if (r >= r1) break;
+        const uint32_t gw[4] = {gv[i].x, gv[i].y, gv[i].z, gv[i].w}, lw[4] = {lv[i].x, lv[i].y, lv[i].z, lv[i].w};
+        uint32_t ow[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 g2 = Cvt<T>::up(gw[e]), l2 = Cvt<T>::up(lw[e]);
+          const float s0 = sigmoid_f(l2.x), s1 = sigmoid_f(l2.y);
+          const float d0 = g2.x * (s0 * (1.f + l2.x * (1.f - s0))), d1 = g2.y * (s1 * (1.f + l2.y * (1.f - s1)));
+          csum[2 * e] += d0;
+          csum[2 * e + 1] += d1;
+          ow[e] = Cvt<T>::down(d0, d1);
+        }
+        *reinterpret_cast<uint4*>(dl + r * p.n) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+      }
     }
-    *reinterpret_cast<uint4*>(&s_t[lr][piece * 8]) = out;
   }
-  // column sums: the 8 lanes that share `piece` across a warp's 4 rows, then the warps of a quarter ... kept simple and
-  // deterministic: every thread adds its two rows, rows are combined through shared memory in a fixed order
-  __shared__ float s_part[32][kBt];
+  // column sums of the block: the warps' sums in a fixed order
 #pragma unroll
-  for (int e = 0; e < 8; ++e) s_part[tid >> 3][piece * 8 + e] = csum[e];
+  for (int e = 0; e < 8; ++e) s_part[warp][lane * 8 + e] = csum[e];
   __syncthreads();
-  if (tid < kBt) {
+  const int c = blockIdx.x * kBtCols + threadIdx.x;
+  if (c < p.n) {
     float acc = 0.f;
-#pragma unroll 8
-    for (int r = 0; r < 32; ++r) acc += s_part[r][tid];
-    if (c0 + tid < p.n) p.partial[static_cast<long long>(blockIdx.y) * p.n + c0 + tid] = acc;
-  }
-  // transposed store: dLT[c][r0 .. r0 + 64) for the 64 columns of the tile, 16 bytes (8 rows) per store
-  for (int i = tid; i < kBt * (kBt / 8); i += kBtThreads) {
-    const int c = i >> 3, rp = (i & 7) * 8;
-    if (c0 + c >= p.n || r0 + rp >= p.ldm) continue;
-    uint32_t w4[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      w4[e] = static_cast<uint32_t>(s_t[rp + 2 * e][c]) | (static_cast<uint32_t>(s_t[rp + 2 * e + 1][c]) << 16);
-    *reinterpret_cast<uint4*>(static_cast<T*>(p.dlt) + static_cast<long long>(c0 + c) * p.ldm + r0 + rp) =
-        make_uint4(w4[0], w4[1], w4[2], w4[3]);
+    for (int r = 0; r < kBtThreads / 32; ++r) acc += s_part[r][threadIdx.x];
+    p.partial[static_cast<long long>(blockIdx.y) * p.n + c] = acc;
   }
 }
 
-// dst [cols, ld_dst] = src [rows, cols]^T for 16-bit elements (cols a multiple of 8, ld_dst a multiple of 8 >= rows).
-__global__ void __launch_bounds__(kBtThreads) transpose16_kernel(const unsigned short* __restrict__ src,
-                                                                  unsigned short* __restrict__ dst, long long rows,
-                                                                  int cols, long long ld_dst) {
-  __shared__ unsigned short s_t[kBt][kBt + 8];
-  const int tid = threadIdx.x;
-  const int c0 = blockIdx.x * kBt;
-  const long long r0 = static_cast<long long>(blockIdx.y) * kBt;
-  for (int i = tid; i < kBt * (kBt / 8); i += kBtThreads) {
-    const int lr = i >> 3, piece = i & 7;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (r0 + lr < rows && c0 + piece * 8 < cols)
-      v = *reinterpret_cast<const uint4*>(src + (r0 + lr) * cols + c0 + piece * 8);
-    *reinterpret_cast<uint4*>(&s_t[lr][piece * 8]) = v;
-  }
-  __syncthreads();
-  for (int i = tid; i < kBt * (kBt / 8); i += kBtThreads) {
-    const int c = i >> 3, rp = (i & 7) * 8;
-    if (c0 + c >= cols || r0 + rp >= ld_dst) continue;
-    uint32_t w4[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      w4[e] = static_cast<uint32_t>(s_t[rp + 2 * e][c]) | (static_cast<uint32_t>(s_t[rp + 2 * e + 1][c]) << 16);
-    *reinterpret_cast<uint4*>(dst + static_cast<long long>(c0 + c) * ld_dst + r0 + rp) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-  }
-}
-
-// bias_grad[c] = sum over the row blocks, in block order
-__global__ void colsum_kernel(const float* __restrict__ partial, float* __restrict__ out, long long blocks, int n) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
+// bias_grad[c] = sum over the row blocks: eight groups of consecutive blocks, each in block order, then the groups
+__global__ void __launch_bounds__(32 * kSumGroups) colsum_kernel(const float* __restrict__ partial, float* __restrict__ out,
+                                                                 long long blocks, int n) {
+  __shared__ float s_sum[kSumGroups][32];
+  const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
+  const long long per = (blocks + kSumGroups - 1) / kSumGroups;
+  const long long b1 = (group + 1) * per < blocks ? (group + 1) * per : blocks;
   float acc = 0.f;
-  for (long long b = 0; b < blocks; ++b) acc += partial[b * n + c];
-  out[c] = acc;
+  if (c < n) {
+#pragma unroll 8
+    for (long long b = group * per; b < b1; ++b) acc += partial[b * n + c];
+  }
+  s_sum[group][lane] = acc;
+  __syncthreads();
+  if (group == 0 && c < n) {
+#pragma unroll
+    for (int i = 1; i < kSumGroups; ++i) acc += s_sum[i][lane];
+    out[c] = acc;
+  }
+}
+
+// Rows per CTA of the element-wise pass: 128, or 32 where that leaves fewer than four CTAs per SM of a B200.
+inline int block_rows(long long m, int n) {
+  const long long ctas = (m + 127) / 128 * ((n + kBtCols - 1) / kBtCols);
+  return ctas < 4 * 148 ? 32 : 128;
 }
 
 inline uint64_t up256(uint64_t x) { return (x + 255) & ~static_cast<uint64_t>(255); }
 
+inline uint64_t max_u64(uint64_t a, uint64_t b) { return a > b ? a : b; }
+
 }  // namespace
 
-// Workspace bytes of the backward for an [m, k] x, [n, k] weight.
+// Workspace bytes of the backward for an [m, k] x, [n, k] weight: dL, the column sums, and (one product after the
+// other) the partial sums of a product that is split along its contraction.
 uint64_t in_linear_silu_bwd_workspace(long long m, int n, int k) {
-  const uint64_t ldm = static_cast<uint64_t>((m + 7) / 8 * 8);
-  return up256(static_cast<uint64_t>(m) * n * 2) + up256(static_cast<uint64_t>(n) * ldm * 2) +
-         up256(static_cast<uint64_t>(k) * n * 2) + up256(static_cast<uint64_t>(k) * ldm * 2) +
-         up256(static_cast<uint64_t>((m + kBt - 1) / kBt) * n * 4);
+  const int rows = block_rows(m, n);
+  return up256(static_cast<uint64_t>(m) * n * 2) + up256(static_cast<uint64_t>((m + rows - 1) / rows) * n * 4) +
+         up256(max_u64(product_partial_bytes(m, k, n), product_partial_bytes(n, k, m)));
 }
 
 // grads: the four output gradients; lo: linear_output; every tensor 16-byte aligned; bias_grad fp32 [n] or null.
@@ -180,51 +173,39 @@ cudaError_t launch_in_linear_silu_bwd(const LinSiluParams& shape, const void* x,
   const long long m = shape.m;
   const int n = shape.n, k = shape.k;
   if (m == 0) return cudaSuccess;
-  const long long ldm = (m + 7) / 8 * 8;
-  char* ws = static_cast<char*>(workspace);
-  void* dl = ws;
-  ws += up256(static_cast<uint64_t>(m) * n * 2);
-  void* dlt = ws;
-  ws += up256(static_cast<uint64_t>(n) * ldm * 2);
-  void* wt = ws;
-  ws += up256(static_cast<uint64_t>(k) * n * 2);
-  void* xt = ws;
-  ws += up256(static_cast<uint64_t>(k) * ldm * 2);
-  float* partial = reinterpret_cast<float*>(ws);
-  const long long row_blocks = (m + kBt - 1) / kBt;
-
   SiluGradParams sp;
+  sp.rows = block_rows(m, n);
+  const long long row_blocks = (m + sp.rows - 1) / sp.rows;
+  if (row_blocks > 65535) return cudaErrorInvalidConfiguration;  // m <= 4 194 240 rows per call
+  char* ws = static_cast<char*>(workspace);
+  sp.dl = ws;
+  ws += up256(static_cast<uint64_t>(m) * n * 2);
+  sp.partial = reinterpret_cast<float*>(ws);
+  ws += up256(static_cast<uint64_t>(row_blocks) * n * 4);
+  float* partial = reinterpret_cast<float*>(ws);
   for (int i = 0; i < 4; ++i) {
     sp.grad[i] = grads[i];
     sp.width[i] = shape.width[i];
   }
   for (int i = 0; i < 5; ++i) sp.start[i] = shape.start[i];
   sp.lo = lo;
-  sp.dl = dl;
-  sp.dlt = dlt;
-  sp.partial = partial;
   sp.m = m;
-  sp.ldm = ldm;
   sp.n = n;
-  const dim3 grid_mn((n + kBt - 1) / kBt, static_cast<unsigned>(row_blocks));
-  if (row_blocks > 65535) return cudaErrorInvalidConfiguration;  // m <= 4 194 240 rows per call
+  const dim3 grid((n + kBtCols - 1) / kBtCols, static_cast<unsigned>(row_blocks));
   if (dtype == HSTU_DTYPE_BF16)
-    silu_grad_kernel<__nv_bfloat16><<<grid_mn, kBtThreads, 0, stream>>>(sp);
+    silu_grad_kernel<__nv_bfloat16><<<grid, kBtThreads, 0, stream>>>(sp);
   else
-    silu_grad_kernel<__half><<<grid_mn, kBtThreads, 0, stream>>>(sp);
+    silu_grad_kernel<__half><<<grid, kBtThreads, 0, stream>>>(sp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  transpose16_kernel<<<dim3((k + kBt - 1) / kBt, (n + kBt - 1) / kBt), kBtThreads, 0, stream>>>(
-      static_cast<const unsigned short*>(weight), static_cast<unsigned short*>(wt), n, k, n);
-  transpose16_kernel<<<dim3((k + kBt - 1) / kBt, static_cast<unsigned>(row_blocks)), kBtThreads, 0, stream>>>(
-      static_cast<const unsigned short*>(x), static_cast<unsigned short*>(xt), m, k, ldm);
-  if (bias_grad) colsum_kernel<<<(n + 255) / 256, 256, 0, stream>>>(partial, bias_grad, row_blocks, n);
-  e = cudaGetLastError();
+  if (bias_grad) {
+    colsum_kernel<<<(n + 31) / 32, 32 * kSumGroups, 0, stream>>>(sp.partial, bias_grad, row_blocks, n);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  // x_grad [m, k] = dL [m, n] . weight [n, k];  weight_grad [n, k] = dL^T . x [m, k]
+  e = launch_product(sp.dl, false, weight, m, k, n, x_grad, partial, dtype, status, stream);
   if (e != cudaSuccess) return e;
-  // x_grad [m, k] = dL [m, n] . (weight^T [k, n])^T ;  weight_grad [n, k] = dLT [n, m] . (x^T [k, m])^T
-  e = launch_gemm_abt(dl, m, n, wt, k, n, n, x_grad, dtype, status, stream);
-  if (e != cudaSuccess) return e;
-  return launch_gemm_abt(dlt, n, ldm, xt, k, ldm, m, weight_grad, dtype, status, stream);
+  return launch_product(sp.dl, true, x, n, k, m, weight_grad, partial, dtype, status, stream);
 }
 
 }  // namespace hstu
