@@ -59,26 +59,21 @@ __device__ __forceinline__ float bias_at(const KParams& p, int b, int h, int i, 
 template <typename T>
 __device__ __forceinline__ void score_grad(const KParams& p, int b, int h, int i, int j, bool visible, float s, float dp,
                                            float bv, float* p_out, float* ds_out, float* dbias_out) {
-  float pv = 0.f, ds = 0.f, db = 0.f;
-  if (visible) {
-    const bool alpha_first = (p.flags & HSTU_FLAG_ALPHA_BEFORE_BIAS) != 0;
-    float x = s;
-    if (p.bias) {
-      x = alpha_first ? fmaf(x, p.alpha, bv) : (x + bv) * p.alpha;
-    } else {
-      x *= p.alpha;
-    }
-    float m = 1.f;
-    if (p.mask_type == HSTU_MASK_CUSTOM) {
-      const long long moff = ((static_cast<long long>(b) * p.hq + h) * p.maxq + i) * p.maxk + j;
-      m = ld_f<T>(static_cast<const T*>(p.mask) + moff);
-    }
-    const float sg = 1.f / (1.f + expf(-x));
-    pv = round_to<T>(x * sg * p.scale * m);
-    const float dx = dp * p.scale * m * sg * (1.f + x * (1.f - sg));
-    ds = round_to<T>(dx * p.alpha);
-    db = alpha_first ? round_to<T>(dx) : ds;
+  // (selects, no branch around the arithmetic: a thread has up to sixteen elements in a row)
+  const bool alpha_first = (p.flags & HSTU_FLAG_ALPHA_BEFORE_BIAS) != 0;
+  float x = s;
+  if (p.bias) x = alpha_first ? fmaf(x, p.alpha, bv) : (x + bv) * p.alpha;
+  else x *= p.alpha;
+  float m = 1.f;
+  if (p.mask_type == HSTU_MASK_CUSTOM && visible) {
+    const long long moff = ((static_cast<long long>(b) * p.hq + h) * p.maxq + i) * p.maxk + j;
+    m = ld_f<T>(static_cast<const T*>(p.mask) + moff);
   }
+  const float sg = simt::divide(1.f, 1.f + expf(-x));
+  const float dx = dp * p.scale * m * sg * (1.f + x * (1.f - sg));
+  const float pv = visible ? round_to<T>(x * sg * p.scale * m) : 0.f;
+  const float ds = visible ? round_to<T>(dx * p.alpha) : 0.f;
+  const float db = visible ? (alpha_first ? round_to<T>(dx) : round_to<T>(dx * p.alpha)) : 0.f;
   *p_out = pv;
   *ds_out = ds;
   *dbias_out = db;
@@ -456,7 +451,7 @@ cudaError_t launch_simt_bwd(const BwdParams& bp, cudaStream_t stream) {
 }
 
 // The register-tiled kernels wherever their loads are possible.  (16 sequences of 50-500 rows, 2 heads of 64, fp32, forward
-// and backward: 191 us, 1239 us with the other kernels.)
+// and backward: 169 us, 1236 us with the other kernels.)
 bool simt_bwd_supported(const BwdParams& bp, int dtype) {
   return simt::dims_ok(bp.f) && simt::aligned_to(bp.f.q, dtype) && simt::aligned_to(bp.f.k, dtype) &&
          simt::aligned_to(bp.f.v, dtype) && simt::aligned_to(bp.dout, dtype) && simt::aligned_to(bp.dq, dtype) &&

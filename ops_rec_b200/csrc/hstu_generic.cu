@@ -100,16 +100,15 @@ __global__ void __launch_bounds__(simt::kThreads) hstu_simt_fwd_kernel(const KPa
 #pragma unroll
         for (int c = 0; c < kCols; ++c) {
           const int i = r0 + 4 * ty + r, j = c0 + tx + 16 * c;
-          float pv = 0.f;
-          if (allowed(rb[r], j)) {
-            float x = sc[r][c];
-            if (bias) x = alpha_first ? fmaf(x, p.alpha, bv[r][c]) : (x + bv[r][c]) * p.alpha;
-            else x *= p.alpha;
-            pv = x / (1.f + expf(-x)) * p.scale;
-            if (p.mask_type == HSTU_MASK_CUSTOM)
-              pv *= to_f<T>(cmask[((static_cast<long long>(b) * p.hq + h) * p.maxq + i) * p.maxk + j]);
-            pv = simt::rounded<T>(pv);
-          }
+          // (no branch per element: sixteen of them in a row were a third of a tile's time)
+          const bool on = allowed(rb[r], j);
+          float x = sc[r][c];
+          if (bias) x = alpha_first ? fmaf(x, p.alpha, bv[r][c]) : (x + bv[r][c]) * p.alpha;
+          else x *= p.alpha;
+          float pv = simt::divide(x, 1.f + expf(-x)) * p.scale;
+          if (p.mask_type == HSTU_MASK_CUSTOM)
+            pv *= on ? to_f<T>(cmask[((static_cast<long long>(b) * p.hq + h) * p.maxq + i) * p.maxk + j]) : 0.f;
+          pv = on ? simt::rounded<T>(pv) : 0.f;
           Ps[(4 * ty + r) * ldp + tx + 16 * c] = pv;
         }
       simt::cp_async_wait<0>();   // V_t

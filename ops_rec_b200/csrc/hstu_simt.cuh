@@ -33,6 +33,16 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(f
 template <> __device__ __forceinline__ __half from_float<__half>(float x) { return __float2half_rn(x); }
 template <typename T> __device__ __forceinline__ float rounded(float x) { return to_float<T>(from_float<T>(x)); }
 
+// a / b (b >= 1) without the slow path of an IEEE division: the reciprocal, and one correction of the quotient from its
+// remainder, which leaves it within an ulp.  (An infinite b or a keeps the uncorrected quotient.)
+__device__ __forceinline__ float divide(float a, float b) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b));
+  const float q = a * r, rem = fmaf(-q, b, a);
+  const float c = fmaf(rem, r, q);
+  return c == c ? c : q;
+}
+
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
