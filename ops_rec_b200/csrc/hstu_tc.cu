@@ -38,16 +38,20 @@
 #include <type_traits>
 
 #include "hstu_common.cuh"
+#include "hstu_tc_common.cuh"
 #include "ptx_sm100.cuh"
 
 namespace hstu {
+
+bool short_preferred(const KParams& p);
+cudaError_t launch_short(const KParams& p, int dtype, const CUtensorMap& mq, const CUtensorMap& mb, int num_sms,
+                         cudaStream_t stream);
 
 namespace {
 
 constexpr int kThreads = 384;
 constexpr int kTmemCols = 512;
 constexpr int kColS0 = 0, kColS1 = 128, kColO0 = 256;
-constexpr long long kWaitLimitCycles = 2000000000ll;  // ~1 s
 constexpr int kSchedStages = 8;                       // depth of the work-item ring between scheduler and roles
 constexpr int kSchedReaders = 3 + 2 * 128;            // producer lane + two MMA lanes + every thread of both P/O groups
                                                       // (+ the two bias cursors of the scheduler thread, kBias == 2)
@@ -118,39 +122,6 @@ struct Barriers {
 };
 static_assert(sizeof(Barriers) <= 2048, "barrier block too large");
 
-// The waiting loop of Waiter::wait, one copy for every wait of the kernel (the fast path - the phase is already
-// complete - stays inline): less code for the instruction caches, and the warps that spin all spin in the same lines.
-__device__ __noinline__ void wait_slow(int* abort_flag, uint32_t* status, uint32_t bar, uint32_t parity) {
-  if (*reinterpret_cast<volatile int*>(abort_flag)) return;
-  const long long t0 = clock64();
-  unsigned spins = 0;
-  while (!ptx::mbar_try_wait(bar, parity)) {
-    if ((++spins & 0x3ffu) == 0) {
-      if (*reinterpret_cast<volatile int*>(abort_flag)) return;
-      if (clock64() - t0 > kWaitLimitCycles) {
-        *reinterpret_cast<volatile int*>(abort_flag) = 1;
-        atomicOr(status, static_cast<uint32_t>(HSTU_ST_PIPE_TIMEOUT));
-        return;
-      }
-    }
-  }
-}
-
-struct Waiter {
-  int* abort_flag;
-  uint32_t* status;
-  // `polled` is the result of an earlier mbar_try_wait on the same phase (polls of several barriers are issued
-  // back to back so that their latencies overlap); only an unsuccessful poll falls into the waiting loop.
-  __device__ __forceinline__ void wait_polled(bool polled, uint32_t bar, uint32_t parity) const {
-    if (!polled) wait(bar, parity);
-  }
-  __device__ __forceinline__ bool aborted() const { return *reinterpret_cast<volatile int*>(abort_flag) != 0; }
-  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) const {
-    if (ptx::mbar_try_wait(bar, parity)) return;
-    wait_slow(abort_flag, status, bar, parity);
-  }
-};
-
 // Consumer side of the work-item ring: every role sees the same sequence of items, in the order the scheduler
 // warp drew them from the global counter.
 struct ItemFeed {
@@ -196,34 +167,6 @@ __device__ __forceinline__ Item load_item(const KParams& p, long long idx) {
   return it;
 }
 
-template <typename T> struct Pack;
-template <> struct Pack<__nv_bfloat16> {
-  static constexpr int kFormat = 1;
-  static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  static __device__ __forceinline__ float2 unpack(uint32_t u) {
-    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
-  }
-  static __device__ __forceinline__ float one(const void* p, long long i) {
-    return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
-  }
-};
-template <> struct Pack<__half> {
-  static constexpr int kFormat = 0;
-  static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
-    __half2 v = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  static __device__ __forceinline__ float2 unpack(uint32_t u) {
-    return __half22float2(*reinterpret_cast<__half2*>(&u));
-  }
-  static __device__ __forceinline__ float one(const void* p, long long i) {
-    return __half2float(static_cast<const __half*>(p)[i]);
-  }
-};
-
 struct BiasRow {
   const void* base;     // attn_bias
   long long row;        // element offset of (b, h, i, 0)
@@ -256,54 +199,6 @@ __device__ __forceinline__ void load_bias32(const BiasRow& br, int jb, uint32_t 
   }
 }
 
-// 32 scores of one row (fp32 bits in sr) -> 16 words of packed P.  Branch-free; the arithmetic runs on the
-// packed f32x2 pipe.  x = c_in * s + c_bias * bias covers both orders of alpha and bias (c_bias = c_in gives
-// alpha * (s + bias)).
-// One tanh.approx per element is the SFU's whole budget (16 results/clk/SM = 1024 clk per 128 x 128 tile).  Moving
-// half of the columns to an FMA-pipe polynomial was tried: it is faster only without a range check, and any
-// data-dependent branch in this block costs more than it saves, so every element goes through the SFU.
-template <typename T, int kBias, bool kMasked>
-__device__ __forceinline__ void silu_chunk(const uint32_t (&sr)[32], const uint32_t (&bv)[16], uint32_t (&pr)[16],
-                                           float c_in, float c_bias, float scale, uint32_t visible) {
-  constexpr bool kExact = Pack<T>::kFormat == 0;  // fp16: exp2 + rcp (two MUFU ops); bf16: tanh form (one)
-  const float2 cin2 = make_float2(c_in, c_in);
-  const float2 cb2 = make_float2(c_bias, c_bias);
-  const float2 sc2 = make_float2(scale, scale);
-#pragma unroll
-  for (int e = 0; e < 16; ++e) {
-    float2 x = make_float2(__uint_as_float(sr[2 * e]), __uint_as_float(sr[2 * e + 1]));
-    if (kBias == 1)
-      x = __ffma2_rn(x, cin2, __fmul2_rn(Pack<T>::unpack(bv[e]), cb2));
-    else
-      x = __fmul2_rn(x, cin2);
-    const float2 r = __fmul2_rn(x, sc2);
-    float2 o;
-    if (kExact) {
-      // sigmoid form: o = y*scale / (1 + 2^(-y log2 e))
-      const float2 ny = __fmul2_rn(x, make_float2(-1.4426950408889634f, -1.4426950408889634f));
-      const float2 d = __fadd2_rn(make_float2(ptx::ex2_approx(ny.x), ptx::ex2_approx(ny.y)), make_float2(1.f, 1.f));
-      o = __fmul2_rn(r, make_float2(ptx::rcp_approx(d.x), ptx::rcp_approx(d.y)));
-    } else {
-      // tanh form on x = y/2: o = x*scale*(1 + tanh x)
-      o = __ffma2_rn(r, make_float2(ptx::tanh_approx(x.x), ptx::tanh_approx(x.y)), r);
-    }
-    if (kBias == 3) o = __fmul2_rn(o, Pack<T>::unpack(bv[e]));  // custom mask: its values multiply (fp32)
-    if (kMasked) {  // a select, not a multiply: scores of rows past the sequence end may be Inf or NaN
-      o.x = (visible & (1u << (2 * e))) ? o.x : 0.f;
-      o.y = (visible & (2u << (2 * e))) ? o.y : 0.f;
-    }
-    pr[e] = Pack<T>::pack(o.x, o.y);
-  }
-}
-
-// Bit e set <=> column j0 + e is visible to the row described by rb (columns j0 .. j0 + 31).
-__device__ __forceinline__ uint32_t low_bits(int n) {  // n lowest bits set, n clamped to [0, 32]
-  return n <= 0 ? 0u : (n >= 32 ? 0xffffffffu : ((1u << n) - 1u));
-}
-__device__ __forceinline__ uint32_t visible_bits(const RowBounds& rb, int j0) {
-  return low_bits(rb.lim1 - j0) | (low_bits(rb.hi2 + 1 - j0) & ~low_bits(rb.lo2 - j0));
-}
-
 // kBias == 2, a sequence's last K tile: the 16-column slice that contains the sequence end is not added by the tensor
 // cores - whatever lies in the bias buffer beyond column lk would reach the slice's visible columns through the
 // identity product (0 x NaN).  The warps that own the slice add its n (< 16) in-sequence bias values of their rows to
@@ -323,14 +218,6 @@ __device__ __forceinline__ void add_end_slice(uint32_t t_slice, const uint32_t (
   }
   ptx::tmem_st16(t_slice, v);
   ptx::tmem_wait_st();
-}
-
-// Zeroes `pieces` 16-byte pieces from shared-memory address `first` on, in each of `boxes` regions `box_bytes` apart
-// (the rows of a V tile behind a sequence end); called by the 128 threads of a P/O group, `tid` = 0..127.
-__device__ __noinline__ void zero_v_rows(uint32_t first, int pieces, int tid, int boxes, int box_bytes) {
-  for (int i = tid; i < pieces; i += kTileM)
-    for (int b = 0; b < boxes; ++b) ptx::st_shared_zero16(first + b * box_bytes + i * 16);
-  ptx::fence_proxy_async();
 }
 
 // This thread's 64 columns of one 128 x 128 score tile, its row: S (TMEM, fp32) -> P (TMEM, packed 16-bit).
@@ -1041,14 +928,14 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// 3-D view (dim, heads, tokens) of a contiguous [tokens, heads, dim] tensor; box = 64 x 1 x 128, 128-byte swizzle.
-bool make_map(CUtensorMap* m, const void* base, long long tokens, int heads, int dim, int dtype) {
+// 3-D view (dim, heads, tokens) of a contiguous [tokens, heads, dim] tensor; box = 64 x 1 x box_rows, 128-byte swizzle.
+bool make_map(CUtensorMap* m, const void* base, long long tokens, int heads, int dim, int dtype, int box_rows = kTileM) {
   auto fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[3] = {static_cast<cuuint64_t>(dim), static_cast<cuuint64_t>(heads),
                         static_cast<cuuint64_t>(tokens > 0 ? tokens : 1)};
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(dim) * 2, static_cast<cuuint64_t>(dim) * 2 * heads};
-  cuuint32_t box[3] = {64, 1, static_cast<cuuint32_t>(kTileM)};
+  cuuint32_t box[3] = {64, 1, static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[3] = {1, 1, 1};
   const CUtensorMapDataType dt = dtype == HSTU_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                           : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -1149,6 +1036,11 @@ bool make_store_map(CUtensorMap* m, void* base, long long rows, long long cols, 
 // The bias tile map (64 x 128 boxes, 128-byte swizzle) for other translation units (the backward kernels).
 bool make_bias_tile_map(CUtensorMap* m, const KParams& p, int dtype) { return make_bias_map(m, p, dtype); }
 
+// The same with boxes of `box_rows` tokens (hstu_short.cu).
+bool make_kv_tile_map(CUtensorMap* m, const void* base, long long tokens, int heads, int dim, int dtype, int box_rows) {
+  return make_map(m, base, tokens, heads, dim, dtype, box_rows);
+}
+
 // The q / k / v tile map for other translation units (the backward kernels).
 bool make_tile_map(CUtensorMap* m, const void* base, long long tokens, int heads, int dim, int dtype) {
   return make_map(m, base, tokens, heads, dim, dtype);
@@ -1194,6 +1086,7 @@ cudaError_t launch_tc(const KParams& p_in, int dtype, int num_sms, cudaStream_t 
       (p.bias_bstride == 0 || p.bias_bstride == static_cast<long long>(p.hq) * p.maxq * p.maxk) &&
       make_bias_map(&mb, p, dtype))
     bias_mode = 2;
+  if ((bias_mode == 0 || bias_mode == 2) && short_preferred(p)) return launch_short(p, dtype, mq, mb, num_sms, stream);
   CUtensorMap mo;
   if (!make_out_map(&mo, p, dtype)) return cudaErrorNotSupported;
   // hstu_paged with direct page reads: the cache as one K / V tensor of num_pages * 2 * 128 rows

@@ -1,0 +1,66 @@
+"""The forward kernel for batches of short sequences (csrc/hstu_short.cu) at the edges of its 64-key and 128-row tiles and of
+the rule that sends calls to it, against the oracle (tolerances of the other parity tests)."""
+import pytest
+import torch
+
+from tests._parity import assert_parity, run_cabi
+from tests._util import make_case
+
+pytestmark = pytest.mark.gpu
+
+BF16, FP16 = torch.bfloat16, torch.float16
+
+
+@pytest.mark.parametrize("dims", [(64, 64), (8, 16), (48, 32)])
+@pytest.mark.parametrize("L", [1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 191, 192, 193, 257, 319])
+@pytest.mark.parametrize("dtype,rab", [(BF16, None), (FP16, "batch"), (BF16, "shared3")])
+def test_lengths(dims, L, dtype, rab):
+    args = make_case(3, 4, 2, *dims, L, L, dtype, seed=L, rab=rab, max_seq_len=(L + 7) // 8 * 8)
+    out, status = run_cabi(args)
+    assert status == 0
+    assert_parity(out, args, label=f"{dims} {L}")
+
+
+@pytest.mark.parametrize("dims", [(128, 128), (72, 80), (64, 128)])
+@pytest.mark.parametrize("lo,hi,kw", [(1, 90, {}), (60, 95, dict(rab="shared3")), (1, 70, dict(mask_type=2)),
+                                      (20, 60, dict(tgt=9, g=2, ctx=3, rab="batch", delta=True))])
+def test_wide(dims, lo, hi, kw):
+    args = make_case(7, 4, 2, *dims, lo, hi, BF16, seed=hi, max_seq_len=96, **kw)
+    out, status = run_cabi(args)
+    assert status == 0
+    assert_parity(out, args, label=f"{dims} {hi}")
+
+
+@pytest.mark.parametrize("rab,tgt", [(None, 5), ("shared3", 0)])
+def test_many_items(rab, tgt):
+    """More work items than eight per CTA: pairs of Q tiles, look-ups spread over the tiles before."""
+    args = make_case(2600, 2, 2, 32, 32, 1, 150, BF16, seed=1, rab=rab, tgt=tgt, g=1 if tgt else 0, max_seq_len=160)
+    out, status = run_cabi(args)
+    assert status == 0
+    assert_parity(out, args)
+
+
+@pytest.mark.parametrize("batch,lo,hi", [(40, 300, 339), (300, 500, 1100), (10, 500, 1100)])
+def test_around_the_rule(batch, lo, hi):
+    """Both sides of the rule's lines give the oracle's result."""
+    args = make_case(batch, 4, 4, 64, 64, lo, hi, BF16, seed=batch)
+    out, status = run_cabi(args)
+    assert status == 0
+    assert_parity(out, args)
+
+
+@pytest.mark.parametrize("poison", [float("nan"), float("inf")])
+@pytest.mark.parametrize("D", [64, 128])
+def test_neighbours_never_leak(poison, D):
+    """Rows of the other sequences may hold anything."""
+    args = make_case(5, 2, 2, D, D, 70, 90, BF16, seed=2)
+    want, _ = run_cabi(args)
+    off = args["seq_offset"].tolist()
+    for n in ("q", "k", "v"):
+        t = args[n].clone()
+        t[:off[2]] = poison
+        t[off[3]:] = poison
+        args[n] = t
+    out, status = run_cabi(args)
+    assert status == 0
+    assert torch.equal(out[off[2]:off[3]], want[off[2]:off[3]])
