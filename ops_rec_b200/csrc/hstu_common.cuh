@@ -70,6 +70,11 @@ struct KParams {
   // rows - goes through the staging tensors
   const void* kv_cache;       // [num_pages, 2, page_size, hk, d]
   int paged_direct;
+  // hstu_paged on hstu_short.cu (page size a multiple of 64, no bias): nothing is staged - the cached keys are read from
+  // the cache, the target rows from the call's own k / v
+  const void* k_new;          // [total_q, hk, d]
+  const void* v_new;
+  int paged_split;
   // backward on the tensor-core kernels only (0 otherwise): `items` holds two tile lists, bwd_cap_q entries for the
   // dQ pass followed by bwd_cap_k for the dK/dV pass; bwd_all_q_tiles: the dQ pass also visits the q-tiles past a
   // sequence's end (they hold rows of grad_bias that must be zeroed)
@@ -112,13 +117,26 @@ HSTU_HD long long load_index(const void* p, int index_bytes, long long i) {
                           : static_cast<long long>(static_cast<const int*>(p)[i]);
 }
 
-HSTU_HD SeqInfo load_seq(const KParams& p, int b) {
+// What the index arrays say about a sequence, as read (the pre-passes read several sequences before they use the first).
+struct SeqRaw {
+  long long q0, q1, k0, k1, c, t;
+};
+HSTU_HD SeqRaw read_seq(const KParams& p, int b) {
+  SeqRaw r;
+  r.q0 = load_index(p.offq, p.index_bytes, b);
+  r.q1 = load_index(p.offq, p.index_bytes, b + 1);
+  r.k0 = load_index(p.offk, p.index_bytes, b);
+  r.k1 = load_index(p.offk, p.index_bytes, b + 1);
+  r.c = p.ctx ? load_index(p.ctx, p.index_bytes, b) : 0;
+  r.t = p.tgt ? load_index(p.tgt, p.index_bytes, b) : 0;
+  return r;
+}
+
+HSTU_HD SeqInfo make_seq(const KParams& p, const SeqRaw& r) {
   SeqInfo s;
-  s.q0 = load_index(p.offq, p.index_bytes, b);
-  long long q1 = load_index(p.offq, p.index_bytes, b + 1);
-  s.k0 = load_index(p.offk, p.index_bytes, b);
-  long long k1 = load_index(p.offk, p.index_bytes, b + 1);
-  long long lq = q1 - s.q0, lk = k1 - s.k0;
+  s.q0 = r.q0;
+  s.k0 = r.k0;
+  long long lq = r.q1 - s.q0, lk = r.k1 - s.k0;
   // Inconsistent inputs (flagged by check_seq) are made harmless here: no row outside [0, total) and no
   // bias/mask element outside its [max_seq_len_q, max_seq_len_k] block is ever addressed.
   if (s.q0 < 0 || s.q0 > p.total_q) { s.q0 = 0; lq = 0; }
@@ -129,25 +147,20 @@ HSTU_HD SeqInfo load_seq(const KParams& p, int b) {
   if (lk > p.maxk) lk = p.maxk;
   s.lq = lq < 0 ? 0 : static_cast<int>(lq);
   s.lk = lk < 0 ? 0 : static_cast<int>(lk);
-  long long c = p.ctx ? load_index(p.ctx, p.index_bytes, b) : 0;
-  long long t = p.tgt ? load_index(p.tgt, p.index_bytes, b) : 0;
-  s.ctx = c < 0 ? 0 : (c > s.lq ? s.lq : static_cast<int>(c));
-  s.tgt = t < 0 ? 0 : (t > s.lq ? s.lq : static_cast<int>(t));
+  s.ctx = r.c < 0 ? 0 : (r.c > s.lq ? s.lq : static_cast<int>(r.c));
+  s.tgt = r.t < 0 ? 0 : (r.t > s.lq ? s.lq : static_cast<int>(r.t));
   if (s.tgt > s.lk) s.tgt = s.lk;
   return s;
 }
+HSTU_HD SeqInfo load_seq(const KParams& p, int b) { return make_seq(p, read_seq(p, b)); }
 
 // Input consistency of one sequence (HSTU_ST_* bits).  The reference does not check these and would read
 // out of bounds (the bias/mask row stride is max_seq_len_k).
-HSTU_HD unsigned check_seq(const KParams& p, int b) {
+HSTU_HD unsigned check_seq(const KParams& p, const SeqRaw& r) {
   unsigned st = 0;
-  long long q0 = load_index(p.offq, p.index_bytes, b), q1 = load_index(p.offq, p.index_bytes, b + 1);
-  long long k0 = load_index(p.offk, p.index_bytes, b), k1 = load_index(p.offk, p.index_bytes, b + 1);
-  if (q1 < q0 || k1 < k0 || q0 < 0 || k0 < 0 || q1 > p.total_q || k1 > p.total_k) st |= HSTU_ST_BAD_OFFSETS;
-  if (q1 - q0 > p.maxq || k1 - k0 > p.maxk) st |= HSTU_ST_LEN_GT_MAX;
-  long long c = p.ctx ? load_index(p.ctx, p.index_bytes, b) : 0;
-  long long t = p.tgt ? load_index(p.tgt, p.index_bytes, b) : 0;
-  if (c < 0 || t < 0 || c + t > q1 - q0 || t > k1 - k0) st |= HSTU_ST_BAD_CTX_TARGET;
+  if (r.q1 < r.q0 || r.k1 < r.k0 || r.q0 < 0 || r.k0 < 0 || r.q1 > p.total_q || r.k1 > p.total_k) st |= HSTU_ST_BAD_OFFSETS;
+  if (r.q1 - r.q0 > p.maxq || r.k1 - r.k0 > p.maxk) st |= HSTU_ST_LEN_GT_MAX;
+  if (r.c < 0 || r.t < 0 || r.c + r.t > r.q1 - r.q0 || r.t > r.k1 - r.k0) st |= HSTU_ST_BAD_CTX_TARGET;
   return st;
 }
 
@@ -189,11 +202,13 @@ HSTU_HD unsigned check_pages(const KParams& p, int b) {
   const long long pages = pg1 - pg0;
   const long long cached = pages > 0 ? (pages - 1) * p.page_size + last : 0;
   if (last < 0 || last > p.page_size || (pages > 0 && last == 0) || cached != (k1 - k0) - t) return HSTU_ST_BAD_PAGES;
+  bool bad = false;   // (no early return: several reads are in flight)
+#pragma unroll 4
   for (long long s = pg0; s < pg1; ++s) {
     const long long pid = load_index(p.page_ids, p.index_bytes, s);
-    if (pid < 0 || pid >= p.num_pages) return HSTU_ST_BAD_PAGES;
+    bad |= pid < 0 || pid >= p.num_pages;
   }
-  return 0;
+  return bad ? HSTU_ST_BAD_PAGES : 0;
 }
 
 // Visibility of row i as column bounds:  allowed(j)  <=>  j < lim1  ||  (lo2 <= j && j <= hi2).
