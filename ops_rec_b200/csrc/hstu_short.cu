@@ -59,8 +59,11 @@ struct ShTile {
   int b, h, hk, r0;   // r0: first row of the Q tile
   int n;              // K tiles it visits
   int valid;          // 0 = end of work
-  int full_tiles;     // hstu_paged with direct page reads: this many leading K / V tiles lie in whole cache pages
-  long long first_slot;
+  // The keys of a sequence are one segment, or - hstu_paged - two: the cached keys [0, split) and the targets
+  // [split, lk).  A tile lies in one segment: tiles j < n_first start at key 64 j, the others at split + 64 (j - n_first).
+  int split, n_first;
+  int pages;            // hstu_paged: pages of the sequence,
+  long long first_slot; //   and the first of them in page_ids
 };
 
 struct ShBars {
@@ -74,10 +77,10 @@ struct ShBars {
 };
 static_assert(sizeof(ShBars) <= 1024, "barrier block too large");
 
-// This thread's 64 scores -> P, in place.  kMasked: the mask or the sequence end cuts through the tile.
+// This thread's 64 scores -> P, in place.  kMasked: the mask or the segment's end (`left` keys away) cuts through the tile.
 template <typename T, bool kBias, bool kMasked>
 __device__ __forceinline__ void short_p(uint32_t t_s, uint32_t bias_row, uint32_t bias_swz, const RowBounds& rb, int c0,
-                                        float c_in, float scale) {
+                                        int left, float c_in, float scale) {
 #pragma unroll
   for (int ch = 0; ch < 2; ++ch) {
     uint32_t sr[32], bv[16], pr[16];
@@ -85,7 +88,7 @@ __device__ __forceinline__ void short_p(uint32_t t_s, uint32_t bias_row, uint32_
     uint32_t vis = 0xffffffffu;
     bool all_on = true, all_off = false;
     if (kMasked) {
-      vis = visible_bits(rb, c0 + ch * 32);
+      vis = visible_bits(rb, c0 + ch * 32) & low_bits(left - ch * 32);
       all_on = __all_sync(0xffffffffu, vis == 0xffffffffu);
       all_off = __all_sync(0xffffffffu, vis == 0u);
     }
@@ -131,7 +134,7 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
     ptx::prefetch_tensormap(&tm_q);
     ptx::prefetch_tensormap(&tm_k);
     ptx::prefetch_tensormap(&tm_v);
-    if (p.paged_direct) ptx::prefetch_tensormap(&tm_cache);
+    if (p.paged_split) ptx::prefetch_tensormap(&tm_cache);
     if (kBias) ptx::prefetch_tensormap(&tm_bias);
     ptx::mbar_init(ptx::smem_u32(&bars->q_full), 1);
     ptx::mbar_init(ptx::smem_u32(&bars->q_free), 1);
@@ -204,7 +207,7 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
         line(p.offk, e_b + 1ll);
         line(p.ctx, e_b);
         line(p.tgt, e_b);
-        if (p.paged_direct) line(p.page_offsets, e_b);
+        if (p.paged_split) line(p.page_offsets, e_b);
       };
       bool second = false;   // the pair's other tile is still to come
       ShTile pair = {};
@@ -230,9 +233,13 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
           t.hk = t.h / p.gqa_ratio;
           t.s = load_seq(p, t.b);
           if (bad) t.s.lq = t.s.lk = 0;
-          if (p.paged_direct)
-            t.full_tiles = (kTileN / kShKeys) * paged_full_tiles(p.offq, p.offk, p.tgt, p.page_offsets, p.index_bytes,
-                                                                 p.total_q, p.num_page_ids, t.b, &t.first_slot);
+          if (p.paged_split) {
+            long long pg0 = load_index(p.page_offsets, p.index_bytes, t.b), pg1 = load_index(p.page_offsets, p.index_bytes, t.b + 1);
+            if (pg0 < 0) pg0 = 0;
+            if (pg1 > p.num_page_ids) pg1 = p.num_page_ids;
+            t.first_slot = pg0;
+            t.pages = pg1 > pg0 ? static_cast<int>(pg1 - pg0) : 0;
+          }
           if (!many) {
             t.r0 += (1 - static_cast<int>(u & 1)) * kTileM;
           } else if (t.r0 + kTileM < t.s.lq) {   // the later tile now, the first one next
@@ -245,13 +252,16 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
             u_next = draw();
           }
         }
-        t.n = kv_tiles_for_rows(t.s, t.r0, kTileM, p.mask_type, kShKeys);
+        const int seen = kv_tiles_for_rows(t.s, t.r0, kTileM, p.mask_type, 1);   // keys [0, seen) are visited
+        t.split = p.paged_split ? t.s.lk - t.s.tgt : t.s.lk;
+        t.n_first = ((seen < t.split ? seen : t.split) + kShKeys - 1) / kShKeys;
+        t.n = t.n_first + (seen > t.split ? (seen - t.split + kShKeys - 1) / kShKeys : 0);
         t.valid = 1;
         return t;
       };
-      // (an id outside the cache reads as zeros: the coordinate lies past the tensor)
-      auto page = [&](const ShTile& t, int tile) -> long long {
-        return tile < t.full_tiles ? load_index(p.page_ids, p.index_bytes, t.first_slot + tile / (kTileN / kShKeys)) : 0;
+      // page `i` of the tile's sequence (-1: the table has none)
+      auto page = [&](const ShTile& t, int i) -> long long {
+        return p.paged_split && i < t.pages ? load_index(p.page_ids, p.index_bytes, t.first_slot + i) : -1;
       };
       uint32_t q_uses = 0, ring_pos = 0, bias_pos = 0;
       if (many) {
@@ -279,12 +289,17 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
           ++q_uses;
           long long pid = 0;
           for (int j = 0; j < t.n; ++j) {
-            const bool from_cache = j < t.full_tiles;
-            const int row = static_cast<int>(t.s.k0) + j * kShKeys;
-            if (from_cache && j % (kTileN / kShKeys) == 0) {
-              pid = pid_next;
-              if (pid < 0 || pid >= p.num_pages) pid = p.num_pages;
-              pid_next = page(t, j + kTileN / kShKeys);
+            const bool from_cache = p.paged_split && j < t.n_first;
+            int row = static_cast<int>(t.s.k0) + j * kShKeys, in_page = 0;
+            if (from_cache) {
+              in_page = (j * kShKeys) % p.page_size;
+              if (in_page == 0) {
+                pid = pid_next;   // (an id outside the cache reads as zeros: the coordinate lies past the tensor)
+                if (pid < 0 || pid >= p.num_pages) pid = p.num_pages;
+                pid_next = page(t, (j * kShKeys) / p.page_size + 1);
+              }
+            } else if (p.paged_split) {
+              row = static_cast<int>(t.s.q0) + t.s.lq - t.s.tgt + (j - t.n_first) * kShKeys;
             }
 #pragma unroll
             for (int kv = 0; kv < 2; ++kv) {
@@ -295,7 +310,7 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
               const int halves = kv == 0 ? halves_qk : halves_v;
               ptx::mbar_expect_tx(full, halves * C::kKvHalf);
               const CUtensorMap* tm = from_cache ? &tm_cache : (kv == 0 ? &tm_k : &tm_v);
-              const int trow = from_cache ? static_cast<int>((pid * 2 + kv) * kTileN) + (j % (kTileN / kShKeys)) * kShKeys : row;
+              const int trow = from_cache ? static_cast<int>((pid * 2 + kv) * p.page_size) + in_page : row;
 #pragma unroll
               for (int hf = 0; hf < C::kHalves; ++hf)
                 if (hf < halves) ptx::tma_load_3d(sm_ring + stage * C::kKvBytes + hf * C::kKvHalf, tm, full, hf * 64, t.hk, trow);
@@ -344,6 +359,7 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
         w.wait(ptx::smem_u32(&bars->item_full[slot]), (k / kShItems) & 1u);
         if (w.aborted()) break;
         const int n = bars->item[slot].n, valid = bars->item[slot].valid, lk = bars->item[slot].s.lk;
+        const int split = bars->item[slot].split, n_first = bars->item[slot].n_first;
         ptx::mbar_arrive(ptx::smem_u32(&bars->item_free[slot]));
         if (!valid) break;
         if (n == 0) continue;
@@ -385,7 +401,8 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
           if (w.aborted()) break;
           ptx::tc_fence_after();
           const uint64_t vbase = kDescV | static_cast<uint64_t>((sm_ring + st * C::kKvBytes) >> 4);
-          const int keys = lk - j * kShKeys;   // (16-key products wholly behind the sequence's end are left out)
+          // (16-key products wholly behind the segment's end are left out)
+          const int keys = j < n_first ? split - j * kShKeys : lk - split - (j - n_first) * kShKeys;
 #pragma unroll
           for (int ks = 0; ks < kShKeys / 16; ++ks)
             ptx::mma_ts_if(ks * 16 < keys ? 1u : 0u, tmem + kShColO, tmem + ks * 8,
@@ -425,6 +442,7 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
       if (stopped()) break;
       const ShTile& in = bars->item[slot];
       const int valid = in.valid, n = in.n, r0 = in.r0, lq = in.s.lq, lk = in.s.lk;
+      const int split = in.split, n_first = in.n_first;
       const int i_row = r0 + row;
       const bool row_ok = i_row < lq;
       RowBounds rb = {0, 1, 0};
@@ -446,11 +464,12 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
       if (!valid) break;
       bool ok = true;
       for (int j = 0; j < n; ++j) {
-        const int c0 = j * kShKeys, rem = lk - c0;
+        const int c0 = j < n_first ? j * kShKeys : split + (j - n_first) * kShKeys;
+        const int rem = (j < n_first ? split : lk) - c0;
         const uint32_t bb = bias_pos % C::kBiasBufs;
         if (kBias) w.wait(ptx::smem_u32(&bars->bias_full[bb]), (bias_pos / C::kBiasBufs) & 1u);
         if (rem < kShKeys && (rem & 15)) {
-          // the V tile holds rows of the next sequence behind this one's end: P is 0 there, but 0 x NaN is not.  The rows
+          // the V tile holds foreign rows behind the segment's end: P is 0 there, but 0 x NaN is not.  The rows
           // up to the next multiple of 16 (at most 120 pieces of 16 bytes per half) are zeroed; the products stop there.
           const uint32_t pos = ring_base + 2u * j + 1u, st = pos % C::kStages;
           w.wait(ptx::smem_u32(&bars->kv_full[st]), (pos / C::kStages) & 1u);
@@ -467,10 +486,10 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
         ++s_uses;
         ptx::tc_fence_after();
         const uint32_t brow = sm_bias + bb * C::kBiasBytes + row * 128, bswz = row & 7;
-        if (c0 + kShKeys <= full_end)
-          short_p<T, kBias, false>(t_s, brow, bswz, rb, c0, c_in, p.scale);
+        if (c0 + kShKeys <= full_end && rem >= kShKeys)
+          short_p<T, kBias, false>(t_s, brow, bswz, rb, c0, rem, c_in, p.scale);
         else
-          short_p<T, kBias, true>(t_s, brow, bswz, rb, c0, c_in, p.scale);
+          short_p<T, kBias, true>(t_s, brow, bswz, rb, c0, rem, c_in, p.scale);
         if (kBias) ptx::fence_proxy_async();   // the bias tile's buffer goes back to TMA: its reads come first
         ptx::tmem_wait_st();
         ptx::tc_fence_before();
@@ -555,25 +574,43 @@ cudaError_t launch_inst(const KParams& p, const CUtensorMap& mq, const CUtensorM
 //            hstu_paged, 16-80 queries per sequence: 512 of mean 1000: 238 -> 184; 64 of 1000: 53 -> 61
 //   D = 128  8700 of mean 60: 649 -> 481; 3500 of mean 150: 460 -> 487; 220 of 2400: 1453 -> 2105
 //            hstu_paged: 2048 of mean 300: 510 -> 433; 512 of 1000: 292 -> 270; 8 of 1000: 38 -> 44
-bool short_preferred(const KParams& p) {
-  if (p.batch <= 0) return false;
+static bool short_rule(const KParams& p, long long mean_k) {
   const bool wide = p.dqk > 64 || p.dv > 64;
-  const long long mean_q = p.total_q / p.batch, mean_k = p.total_k / p.batch;
+  const long long mean_q = p.total_q / p.batch;
   if (mean_k < (wide ? 96 : 320)) return true;
   const long long tiles = p.hq * (p.total_q / kTileM > p.batch ? p.total_q / kTileM : p.batch);
   if (tiles < kFewItems) return false;
   return mean_q < 96 || (!wide && mean_k < 1024);
+}
+bool short_preferred(const KParams& p) {
+  if (p.paged_split) return true;                     // (decided by short_paged_split)
+  if (p.batch <= 0 || p.paged_direct) return false;   // (cache pages beside staging tensors: hstu_tc.cu)
+  return short_rule(p, p.total_k / p.batch);
+}
+
+// Whether an hstu_paged call can run here without staging anything: K / V tiles of 64 keys lie in one page, and no bias - a
+// bias tile of the targets would start at any column, TMA wants multiples of 16 bytes.
+bool short_paged_split(const KParams& p) {
+  const uintptr_t align = reinterpret_cast<uintptr_t>(p.kv_cache) | reinterpret_cast<uintptr_t>(p.k_new) |
+                          reinterpret_cast<uintptr_t>(p.v_new);
+  if (p.batch <= 0 || p.mask_type == HSTU_MASK_CUSTOM || p.bias || p.page_size % kShKeys != 0 || (align & 15u) != 0 ||
+      p.num_pages > 0x7fffff00ll / 2 / p.page_size)
+    return false;
+  // (the cached keys are not known here: all pages, each sequence's last one half full)
+  return short_rule(p, (p.num_page_ids * p.page_size + p.total_q) / p.batch - p.page_size / 2);
 }
 
 // Returns cudaSuccess, a CUDA error, or cudaErrorNotSupported when a tensor map could not be encoded.
 cudaError_t launch_short(const KParams& p, int dtype, const CUtensorMap& mq, const CUtensorMap& mb, int num_sms,
                          cudaStream_t stream) {
   CUtensorMap mk, mv, mbs = mb;
-  if (!make_kv_tile_map(&mk, p.k, p.total_k, p.hk, p.dqk, dtype, kShKeys) ||
-      !make_kv_tile_map(&mv, p.v, p.total_k, p.hk, p.dv, dtype, kShKeys))
+  const long long rows = p.paged_split ? p.total_q : p.total_k;
+  if (!make_kv_tile_map(&mk, p.paged_split ? p.k_new : p.k, rows, p.hk, p.dqk, dtype, kShKeys) ||
+      !make_kv_tile_map(&mv, p.paged_split ? p.v_new : p.v, rows, p.hk, p.dv, dtype, kShKeys))
     return cudaErrorNotSupported;
   CUtensorMap mc = mk;
-  if (p.paged_direct && !make_kv_tile_map(&mc, p.kv_cache, p.num_pages * 2 * kTileN, p.hk, p.dqk, dtype, kShKeys))
+  if (p.paged_split &&
+      !make_kv_tile_map(&mc, p.kv_cache, p.num_pages * 2 * p.page_size, p.hk, p.dqk, dtype, kShKeys))
     return cudaErrorNotSupported;
 #define HSTU_SHORT_CASE(DD, TT)                                                     \
   return p.bias ? launch_inst<DD, TT, true>(p, mq, mk, mv, mbs, mc, num_sms, stream) \

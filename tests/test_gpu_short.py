@@ -3,8 +3,11 @@ the rule that sends calls to it, against the oracle (tolerances of the other par
 import pytest
 import torch
 
+from oracle import hstu_paged_oracle as PO
+from ops_rec_b200 import cabi
 from tests._parity import assert_parity, run_cabi
 from tests._util import make_case
+from tests.test_paged import make_paged_case
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +67,25 @@ def test_neighbours_never_leak(poison, D):
     out, status = run_cabi(args)
     assert status == 0
     assert torch.equal(out[off[2]:off[3]], want[off[2]:off[3]])
+
+
+@pytest.mark.parametrize("page", [64, 128, 192, 256])
+@pytest.mark.parametrize("D", [64, 32])
+@pytest.mark.parametrize("hist,cand", [(63, 1), (64, 64), (65, 70), (130, 130)])
+def test_paged_without_staging(page, D, hist, cand):
+    """Pages read where they lie, targets from the call's own k / v: both segments' ends fall anywhere in a 64-key tile, and
+    the unused rows of the cache hold NaNs."""
+    args = make_paged_case(12, 4, 2, D, hist, cand, page, True, BF16, seed=hist + page)
+    cache = args["kv_cache"].clone()
+    used = torch.zeros(cache.shape[0], page, dtype=torch.bool)
+    for b in range(len(args["last_page_len"])):
+        ids = args["page_ids"][args["page_offsets"][b]:args["page_offsets"][b + 1]]
+        for i, pid in enumerate(ids.tolist()):
+            used[pid, :page if i + 1 < len(ids) else int(args["last_page_len"][b])] = True
+    cache.transpose(1, 2)[~used] = float("nan")
+    want = PO.hstu_paged_forward(**args, round_p=False, out_dtype=torch.float32)
+    got, status = cabi.hstu_paged_forward(**{k: (v.cuda() if isinstance(v, torch.Tensor) else v)
+                                             for k, v in dict(args, kv_cache=cache).items()}, return_status=True)
+    assert status == 0
+    torch.testing.assert_close(got.float().cpu(), want, rtol=1e-2, atol=1e-2)
+    assert (got.float().cpu() - want).abs().max() <= 2e-2 * want.abs().max()
