@@ -11,7 +11,7 @@
 // needs 1 byte per 64 FLOPs (measured: 531 TFLOP/s, the L2 limit), a 256 x 256 tile half of that.  Shared by a pair, the
 // tile takes half of each CTA's tensor memory, so there are two of them: the epilogue of one tile runs under the main
 // loop of the next.  In each CTA:
-//   warp 0   TMA producer: 64-wide K chunks of this CTA's 128 rows of x and 128 rows of the weight, a 6-stage ring; the
+//   warp 0   TMA producer: 64-wide K chunks of this CTA's 128 rows of x and 128 rows of the weight, a 5-stage ring; the
 //            bytes of both CTAs are counted on the leader's barrier
 //   warp 1   MMA issuer (of the leader, rank 0): tcgen05.mma cta_group::2, M256 N256 K16, fp32 accumulators in TMEM
 //            (each CTA its 128 rows x 256 columns)
@@ -39,7 +39,7 @@ namespace {
 constexpr int kLsThreads = 384;
 constexpr int kLsTile = 256;                    // tile edge of a CTA pair
 constexpr int kLsHalf = 128;                    // each CTA's rows of A and of B
-constexpr int kLsStages = 6;
+constexpr int kLsStages = 5;
 constexpr int kLsChunkBytes = kLsHalf * 128;    // 128 x 64 16-bit values of one operand
 constexpr int kLsPairs = 74;                    // CTA pairs of a B200 (148 SMs): what a product is split for
 constexpr long long kLsWaitLimit = 2000000000ll;
@@ -101,7 +101,7 @@ __device__ __forceinline__ void ls_wait(LsBars* bars, uint32_t* status, uint32_t
   }
 }
 
-constexpr int kLsStageBytes = 8 * 2 * 2048;   // per epilogue warp: 32 rows x 32 columns of linear_output and of SiLU
+constexpr int kLsStageBytes = 8 * 2 * 4096;   // per epilogue warp, twice: 32 rows x 32 columns of linear_output and of SiLU
 constexpr int kLsRingBytes = kLsStages * 2 * kLsChunkBytes;
 
 // kForward: the operator itself, A = x and B = weight, both K-major.  The other modes are bare products for the backward
@@ -248,14 +248,12 @@ in_linear_silu_kernel(const LinSiluParams p, const __grid_constant__ CUtensorMap
     // Each warp turns 32 rows x 32 columns at a time: TMEM -> registers -> (+ bias, round, SiLU) -> its staging block
     // -> TMA stores (one 32-column box of linear_output, 64-byte swizzle; the SiLU values as two 16-column boxes,
     // because a split boundary may fall between them).  The TMEM load of the next 32 columns is in flight while the
-    // current ones are computed; the staging block is reused once the stores of the previous round have read it.
+    // current ones are computed; two staging blocks, so a round does not wait for the previous round's stores.
     const int colh = ((warp - 4) >> 2) * kLsHalf;   // this warp's columns of the tile: [colh, colh + 128)
     const uint32_t lane_base = (static_cast<uint32_t>((warp & 3) * 32) << 16) + colh;
-    const uint32_t st_lin = base + kLsRingBytes + (warp - 4) * 4096;   // 32 rows x 64 bytes, 64-byte swizzle
-    const uint32_t st_act = st_lin + 2048;                            // 2 x (32 rows x 32 bytes)
     const uint32_t swz = (lane >> 1) & 3;      // 64-byte swizzle: 16-byte chunk index ^ address bits [7, 9)
     const int etid = tid - 128;                // 0..255 among the epilogue threads
-    uint32_t it = 0;
+    uint32_t it = 0, round = 0;   // round: 32-column chunks this warp has staged
     for (long long u = pair0; u < units; u += pairs, ++it) {
       const long long t = u / splits;
       const int n0 = static_cast<int>(t % n_tiles) * kLsTile;
@@ -295,6 +293,8 @@ in_linear_silu_kernel(const LinSiluParams p, const __grid_constant__ CUtensorMap
           const int ch = ch2 + u2;
           if (ch >= nch) break;
           const int c0 = n0 + colh + ch * 32;
+          const uint32_t st_lin = base + kLsRingBytes + ((warp - 4) * 2 + (round & 1u)) * 4096;   // 32 rows x 64 bytes, 64-byte swizzle
+          const uint32_t st_act = st_lin + 2048;                                        // 2 x (32 rows x 32 bytes)
           ptx::tmem_wait_ld_dep(acc[u2]);
           if (ch + 1 < nch) ptx::tmem_ld32(src + (ch + 1) * 32, acc[u2 ^ 1]);
           else release();
@@ -319,8 +319,8 @@ in_linear_silu_kernel(const LinSiluParams p, const __grid_constant__ CUtensorMap
             lin[e] = LsPack<T>::pack(sum.x, sum.y);
             if (!kPlain) act[e] = LsPack<T>::silu2(LsPack<T>::unpack(lin[e]));   // SiLU of the rounded value
           }
-          // the stores of the previous round have read the staging block
-          if (lane < 3) ptx::bulk_wait_read<0>();   // (lanes 0..2 issue one store each)
+          // the stores that last used this staging block (two rounds ago: at most the latest one may still be reading)
+          if (lane < 3) ptx::bulk_wait_read<1>();   // (lanes 0..2 issue one store each)
           __syncwarp();
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -335,22 +335,21 @@ in_linear_silu_kernel(const LinSiluParams p, const __grid_constant__ CUtensorMap
           ptx::fence_proxy_async();
           __syncwarp();
           // three lanes issue one store each (an issue costs its thread ~100 cycles); rows and columns past the
-          // matrix edge are clipped by the tensor maps
-          if (row0 < p.m) {
-            if (lane == 0) {
+          // matrix edge are clipped by the tensor maps.  Every round commits a group, an empty one too: the wait above
+          // counts rounds.
+          if (lane < 3) {
+            const int cg = c0 + 16 * (lane - 1);   // the 16-column group decides the SiLU output tensor (n, splits: multiples of 16)
+            const bool rows = row0 < p.m;
+            if (rows && lane == 0) {
               ptx::tma_store_2d(&tm_lin, st_lin, c0, static_cast<int>(row0));
-              ptx::bulk_commit();
-            } else if (!kPlain && lane < 3) {
-              const int hf = lane - 1;
-              const int cg = c0 + 16 * hf;   // the 16-column group decides the SiLU output tensor (n, splits: multiples of 16)
-              if (cg < p.n) {
-                const int which = (cg >= p.start[1]) + (cg >= p.start[2]) + (cg >= p.start[3]);
-                const CUtensorMap* tm = which == 0 ? &tm_o0 : which == 1 ? &tm_o1 : which == 2 ? &tm_o2 : &tm_o3;
-                ptx::tma_store_2d(tm, st_act + hf * 1024, cg - p.start[which], static_cast<int>(row0));
-                ptx::bulk_commit();
-              }
+            } else if (rows && lane > 0 && !kPlain && cg < p.n) {
+              const int which = (cg >= p.start[1]) + (cg >= p.start[2]) + (cg >= p.start[3]);
+              const CUtensorMap* tm = which == 0 ? &tm_o0 : which == 1 ? &tm_o1 : which == 2 ? &tm_o2 : &tm_o3;
+              ptx::tma_store_2d(tm, st_act + (lane - 1) * 1024, cg - p.start[which], static_cast<int>(row0));
             }
+            ptx::bulk_commit();
           }
+          ++round;
         }
       }
     }
