@@ -506,10 +506,9 @@ def run_paged(args, local_rank):
                                f"history rows per user as queries", "query_tokens": tq,
                    "kv_rows": int((cache_len + T).sum()), "l2": f"{nbytes / 1e6:.0f} MB per step: no flush"},
         "roofline": {"bound": "hbm", "achieved": gbs, "peak": peaks["hbm"], "unit": "GB/s", "frac": gbs / peaks["hbm"],
-                     "traffic": None, "kernel": "hstu_paged_gather_kernel + hstu_tc_kernel",
-                     "algorithmic_bytes_per_launch": nbytes, "note": "the gather pass moves the K/V rows a second time "
-                     "(staging write + read), which the algorithmic bytes do not count"},
-        "gpu_launches": 4 * args.steps, "clocks": clocks.summary()}), flush=True)
+                     "traffic": None, "kernel": "hstu_short_kernel", "algorithmic_bytes_per_launch": nbytes,
+                     "note": "cache pages and new rows are read where they lie: pre-pass + one kernel per call"},
+        "gpu_launches": 2 * args.steps, "clocks": clocks.summary()}), flush=True)
 
 
 def run_backward(args, ops_rec, W, full, mine, kw, dev, rank, world, local_rank, warmup, barrier):

@@ -18,16 +18,19 @@
 // TMEM, an element-wise stage by 256 threads (thread = TMEM lane = row, two groups share the columns) that writes
 // the 16-bit results in place over the fp32 ones, and accumulate products (A operand = those results in TMEM, B =
 // the streamed tile again, read N-major).  TMEM: T1, T2 (128 columns each), Acc1, Acc2 (D columns each).
-// A step's element-wise stage and the MMAs do not overlap yet (one chain per CTA); the element-wise math follows
+// The element-wise stage is split where its inputs are: P and the factor of dS need the scores only and are computed
+// while the dP product runs (dK/dV pass: and dV, and the next step's scores, behind P); dS is then one product per
+// element.  (12 sequences of 4096, 8 heads of 128: dQ pass 698 us, dK/dV pass 836 us; the
+// element-wise stage - 1 640 + 810 cycles of a dQ step - is what a step takes now.)  The math follows
 // hstu_backward_v1/op_kernel/vector_score.h:159-209 with P and dS rounded to the input type.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets HSTU_ST_PIPE_TIMEOUT and a CTA-wide abort flag, the
 // kernel still drains its TMA loads, frees its tensor memory and returns.
 #include <cuda.h>
-
-#include <type_traits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "hstu_common.cuh"
 #include "ptx_sm100.cuh"
@@ -72,9 +75,12 @@ template <> struct BPack<__half> {
 
 struct BwdBars {
   uint64_t a_full;             // the resident pair has landed
-  uint64_t b_full[2], b_free[2];
-  uint64_t t_full;             // T1 and T2 of the current step are complete
-  uint64_t u_full[2];          // their 16-bit replacements are written: first / second 32 values of each 64 (256 arrivals)
+  uint64_t b1_full[3], b1_free[3];   // the streamed tiles, a ring each
+  uint64_t b2_full[3], b2_free[3];
+  uint64_t t1_full[2];         // T1 (the scores) of an even / odd step is complete
+  uint64_t t2_full;            // T2 (dP) of the current step is complete
+  uint64_t p_full[2];          // dK/dV pass: P is written, first / second 32 values of each 64 (256 arrivals)
+  uint64_t u_full[2];          // the same for dS
   uint64_t acc_full;           // every accumulate MMA is complete
   uint64_t bias_full, bias_free;   // dK/dV pass with a staged bias tile: landed / read by all 256 element-wise threads
   uint32_t tmem_base;
@@ -132,42 +138,50 @@ __device__ __forceinline__ uint32_t visible_bits(const RowBounds& rb, int j0) {
   return low_bits(rb.lim1 - j0) | (low_bits(rb.hi2 + 1 - j0) & ~low_bits(rb.lo2 - j0));
 }
 
-// P and dS of two neighbouring elements from s = q.k and dp = dO.v (vector_score.h:175-197) on the packed f32x2
-// pipe:  x = alpha (s + bias),  sg = sigmoid(x),  P = x sg scale,  dS = dp scale alpha sg (1 + x - x sg).
-// kSelect: zero the elements whose bit in `vis` (bits 0 and 1) is clear - a select, never a multiply: scores of
-// rows past a sequence end may be Inf or NaN.
+// Two neighbouring elements, the part that needs the scores only (vector_score.h:175-197), on the packed f32x2 pipe:
+//   x = alpha (s + bias),  sg = sigmoid(x),  P = x sg scale,  f = scale alpha sg (1 + x - x sg)   (dS = dP f)
+// With h = x / 2 and th = tanh h:  sg = (1 + th) / 2,  P = scale (h + h th),  f = (scale alpha / 2) (1 + th) (1 + h - h th).
+// kSelect: zero the P whose bit in `vis` (bits 0 and 1) is clear - a select, never a multiply: scores of rows past a
+// sequence end may be Inf or NaN (dS is selected when it is formed).
 template <typename T, bool kBiasOn, bool kSelect>
-__device__ __forceinline__ void score_grad2(float2 s, float2 dp, float2 bias, float alpha, float scale, uint32_t vis,
-                                            uint32_t& p_out, uint32_t& ds_out) {
-  const float2 al = make_float2(alpha, alpha);
-  float2 x = kBiasOn ? __fmul2_rn(__fadd2_rn(s, bias), al) : __fmul2_rn(s, al);
-  float2 sg;
-  if (BPack<T>::kFormat == 0) {
+__device__ __forceinline__ float2 score_part(float2 s, float2 bias, float alpha, float scale, uint32_t vis, uint32_t& p_out) {
+  if (kBiasOn) s = __fadd2_rn(s, bias);
+  float2 pv, f;
+  if (BPack<T>::kFormat == 0) {   // fp16: exp2 and reciprocal
+    const float2 x = __fmul2_rn(s, make_float2(alpha, alpha));
     const float2 ny = __fmul2_rn(x, make_float2(-1.4426950408889634f, -1.4426950408889634f));
     const float2 d = __fadd2_rn(make_float2(ptx::ex2_approx(ny.x), ptx::ex2_approx(ny.y)), make_float2(1.f, 1.f));
-    sg = make_float2(ptx::rcp_approx(d.x), ptx::rcp_approx(d.y));
+    const float2 sg = make_float2(ptx::rcp_approx(d.x), ptx::rcp_approx(d.y));
+    const float2 xs = __fmul2_rn(x, sg);
+    pv = __fmul2_rn(xs, make_float2(scale, scale));
+    const float2 wgt = __ffma2_rn(xs, make_float2(-1.f, -1.f), __fadd2_rn(x, make_float2(1.f, 1.f)));
+    f = __fmul2_rn(__fmul2_rn(sg, make_float2(scale * alpha, scale * alpha)), wgt);
   } else {
-    const float2 hx = __fmul2_rn(x, make_float2(0.5f, 0.5f));
-    sg = __ffma2_rn(make_float2(ptx::tanh_approx(hx.x), ptx::tanh_approx(hx.y)), make_float2(0.5f, 0.5f),
-                    make_float2(0.5f, 0.5f));
+    const float2 h = __fmul2_rn(s, make_float2(0.5f * alpha, 0.5f * alpha));
+    const float2 th = make_float2(ptx::tanh_approx(h.x), ptx::tanh_approx(h.y));
+    const float c = 0.5f * scale * alpha;
+    const float2 ht = __fmul2_rn(h, th);
+    pv = __fmul2_rn(__fadd2_rn(h, ht), make_float2(scale, scale));
+    const float2 wgt = __ffma2_rn(ht, make_float2(-1.f, -1.f), __fadd2_rn(h, make_float2(1.f, 1.f)));
+    f = __fmul2_rn(__ffma2_rn(th, make_float2(c, c), make_float2(c, c)), wgt);
   }
-  const float2 xs = __fmul2_rn(x, sg);
-  float2 pv = __fmul2_rn(xs, make_float2(scale, scale));
-  const float2 wgt = __ffma2_rn(xs, make_float2(-1.f, -1.f), __fadd2_rn(x, make_float2(1.f, 1.f)));
-  const float sa = scale * alpha;
-  float2 ds = __fmul2_rn(__fmul2_rn(__fmul2_rn(dp, make_float2(sa, sa)), sg), wgt);
   if (kSelect) {
     pv.x = (vis & 1u) ? pv.x : 0.f;
     pv.y = (vis & 2u) ? pv.y : 0.f;
-    ds.x = (vis & 1u) ? ds.x : 0.f;
-    ds.y = (vis & 2u) ? ds.y : 0.f;
   }
   p_out = BPack<T>::pack(pv.x, pv.y);
-  ds_out = BPack<T>::pack(ds.x, ds.y);
+  return f;
 }
 
 // kStaged (dK/dV pass with a bias that TMA can tile): a kernel of its own - the same code merely present in the
 // bias-free kernel cost that one 4 %.
+template <int D, bool kStaged, bool kDKV> struct BwdRings {
+  static constexpr int k1 = kDKV || (D == 128 && kStaged) ? 2 : 3, k2 = 2;
+  static constexpr int kSmem = 1024 + (2 + k1 + k2) * (D / 64) * kTileM * 128 + (kStaged ? 2 * kTileM * 128 : 0) + 512;
+  static_assert(kSmem <= 232448, "shared memory budget of one CTA exceeded");
+};
+static_assert(sizeof(BwdBars) <= 512, "barrier block too large");
+
 template <int D, typename T, bool kDKV, bool kStaged>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1,
@@ -192,13 +206,18 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t sm_a = base;                        // A1, A2
-  const uint32_t sm_b = base + 2 * kTileBytes;       // ring: stage x {B1, B2}
+  // Rings of the streamed tiles B1 (read by the scores and by the last products of a step) and B2 (dQ pass: by dP only).
+  // With two slots of B1 the loads of step c + 1 can start when step c - 1 has ended - in the dQ pass too late by 600 cycles
+  // a step: three there, wherever the shared memory has room (not at D = 128 beside a staged bias tile).  The dK/dV pass,
+  // whose steps are longer, did not gain (838 -> 855 us on the batch above).
+  constexpr uint32_t kRing1 = BwdRings<D, kStaged, kDKV>::k1, kRing2 = BwdRings<D, kStaged, kDKV>::k2;
+  const uint32_t sm_b1 = base + 2 * kTileBytes, sm_b2 = sm_b1 + kRing1 * kTileBytes;
   // With a bias that TMA can tile: the 128 x 128 bias tile of a step (rows = queries, columns = keys), staged by TMA.
   // dK/dV pass: a thread owns a key and reads its column, one value per query, from shared memory instead of 32
   // strided 2-byte loads from global memory per chunk; dQ pass: a thread owns a query and reads 64 bytes of its row
-  const uint32_t sm_bias = base + 6 * kTileBytes;    // 2 boxes of 128 rows x 128 bytes, 128-byte swizzle
+  const uint32_t sm_bias = sm_b2 + kRing2 * kTileBytes;    // 2 boxes of 128 rows x 128 bytes, 128-byte swizzle
   constexpr bool staged = kStaged;
-  BwdBars* bars = reinterpret_cast<BwdBars*>(base_ptr + 6 * kTileBytes + (staged ? 2 * kTileM * 128 : 0));
+  BwdBars* bars = reinterpret_cast<BwdBars*>(base_ptr + (2 + kRing1 + kRing2) * kTileBytes + (staged ? 2 * kTileM * 128 : 0));
   const BwdWaiter w{&bars->abort_flag, p.ws_header};
 
   // The two passes do not depend on each other, only on the pre-pass before them.  The dK/dV pass is launched with
@@ -214,13 +233,18 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
     ptx::prefetch_tensormap(&tm_b1);
     ptx::prefetch_tensormap(&tm_b2);
     ptx::mbar_init(ptx::smem_u32(&bars->a_full), 1);
-    for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(ptx::smem_u32(&bars->b_full[i]), 1);
-      ptx::mbar_init(ptx::smem_u32(&bars->b_free[i]), 1);
+    for (int i = 0; i < 3; ++i) {
+      ptx::mbar_init(ptx::smem_u32(&bars->b1_full[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&bars->b1_free[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&bars->b2_full[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&bars->b2_free[i]), 1);
     }
-    ptx::mbar_init(ptx::smem_u32(&bars->t_full), 1);
-    ptx::mbar_init(ptx::smem_u32(&bars->u_full[0]), 2 * kTileM);
-    ptx::mbar_init(ptx::smem_u32(&bars->u_full[1]), 2 * kTileM);
+    ptx::mbar_init(ptx::smem_u32(&bars->t2_full), 1);
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(ptx::smem_u32(&bars->t1_full[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&bars->p_full[i]), 2 * kTileM);
+      ptx::mbar_init(ptx::smem_u32(&bars->u_full[i]), 2 * kTileM);
+    }
     ptx::mbar_init(ptx::smem_u32(&bars->acc_full), 1);
     ptx::mbar_init(ptx::smem_u32(&bars->bias_full), 1);
     ptx::mbar_init(ptx::smem_u32(&bars->bias_free), 2 * kTileM);
@@ -306,8 +330,19 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
           if (hf < halves2) ptx::tma_load_3d(sm_a + kTileBytes + hf * kHalfBytes, &tm_a2, afull, hf * 64, a_head, static_cast<int>(a_row));
         }
         for_each_step<kDKV>(p, s, tile0, head, [&](int sh, int srow0, int qh) {
-          const uint32_t stage = cnt & 1u;
-          const uint32_t full = ptx::smem_u32(&bars->b_full[stage]);
+          const int row = static_cast<int>(b_row0) + srow0;
+          const uint32_t s1 = cnt % kRing1, s2 = cnt % kRing2;
+          const uint32_t full1 = ptx::smem_u32(&bars->b1_full[s1]), full2 = ptx::smem_u32(&bars->b2_full[s2]);
+          w.wait(ptx::smem_u32(&bars->b1_free[s1]), ((cnt / kRing1) & 1u) ^ 1u);
+          ptx::mbar_expect_tx(full1, halves1 * kHalfBytes);
+#pragma unroll
+          for (int hf = 0; hf < kHalves; ++hf)
+            if (hf < halves1) ptx::tma_load_3d(sm_b1 + s1 * kTileBytes + hf * kHalfBytes, &tm_b1, full1, hf * 64, sh, row);
+          w.wait(ptx::smem_u32(&bars->b2_free[s2]), ((cnt / kRing2) & 1u) ^ 1u);
+          ptx::mbar_expect_tx(full2, halves2 * kHalfBytes);
+#pragma unroll
+          for (int hf = 0; hf < kHalves; ++hf)
+            if (hf < halves2) ptx::tma_load_3d(sm_b2 + s2 * kTileBytes + hf * kHalfBytes, &tm_b2, full2, hf * 64, sh, row);
           if (staged) {
             // the bias tile of this step, once every element-wise thread has read the last one
             w.wait(ptx::smem_u32(&bars->bias_free), (cnt & 1u) ^ 1u);
@@ -320,14 +355,6 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
             for (int hf = 0; hf < 2; ++hf)
               ptx::tma_load_2d(sm_bias + hf * (kTileM * 128), &tm_bias, bfull, bcol0 + hf * 64, brow);
           }
-          w.wait(ptx::smem_u32(&bars->b_free[stage]), ((cnt >> 1) & 1u) ^ 1u);
-          ptx::mbar_expect_tx(full, (halves1 + halves2) * kHalfBytes);
-          const int row = static_cast<int>(b_row0) + srow0;
-#pragma unroll
-          for (int hf = 0; hf < kHalves; ++hf) {
-            if (hf < halves1) ptx::tma_load_3d(sm_b + stage * 2 * kTileBytes + hf * kHalfBytes, &tm_b1, full, hf * 64, sh, row);
-            if (hf < halves2) ptx::tma_load_3d(sm_b + stage * 2 * kTileBytes + kTileBytes + hf * kHalfBytes, &tm_b2, full, hf * 64, sh, row);
-          }
           ++cnt;
         });
         ++tiles_done;
@@ -335,10 +362,15 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
       if (tiles_done > 0) {
         // drain (matters only after an abort: otherwise the consumers have waited for every load)
         for (int spin = 0; spin < (1 << 22) && !ptx::mbar_try_wait(ptx::smem_u32(&bars->a_full), (tiles_done - 1) & 1u); ++spin) {}
-        for (uint32_t back = 0; back < 2 && back < cnt; ++back) {
+        for (uint32_t back = 0; back < kRing1 && back < cnt; ++back) {
           const uint32_t c = cnt - 1 - back;
-          const uint32_t bar = ptx::smem_u32(&bars->b_full[c & 1u]);
-          for (int spin = 0; spin < (1 << 22) && !ptx::mbar_try_wait(bar, (c >> 1) & 1u); ++spin) {}
+          const uint32_t bar = ptx::smem_u32(&bars->b1_full[c % kRing1]);
+          for (int spin = 0; spin < (1 << 22) && !ptx::mbar_try_wait(bar, (c / kRing1) & 1u); ++spin) {}
+        }
+        for (uint32_t back = 0; back < kRing2 && back < cnt; ++back) {
+          const uint32_t c = cnt - 1 - back;
+          const uint32_t bar = ptx::smem_u32(&bars->b2_full[c % kRing2]);
+          for (int spin = 0; spin < (1 << 22) && !ptx::mbar_try_wait(bar, (c / kRing2) & 1u); ++spin) {}
         }
         if (staged && cnt > 0)
           for (int spin = 0; spin < (1 << 22) && !ptx::mbar_try_wait(ptx::smem_u32(&bars->bias_full), (cnt - 1) & 1u); ++spin) {}
@@ -402,21 +434,18 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
       constexpr uint64_t kDescN = ptx::umma_desc_sw128_hi(kHalfBytes, 1024);   // the same tiles read N-major
       const uint64_t a1 = kDescK | static_cast<uint64_t>(sm_a >> 4);
       const uint64_t a2 = kDescK | static_cast<uint64_t>((sm_a + kTileBytes) >> 4);
-      // accumulate products of step c (its U1 / U2 are written): Acc1 += U1.B2, Acc2 += U2.B1
-      // The element-wise groups hand their results over in two parts (values 0..31 and 64..95 of a tile row, then
-      // the rest), so the first half of these MMAs runs while the second part is still being computed.
+      // Accumulate products of step c: Acc1 += P.B2 (dK/dV pass), Acc2 += dS.B1.  The element-wise groups hand P and dS over
+      // in two parts each (values 0..31 and 64..95 of a tile row, then the rest), so the first half of these MMAs runs
+      // while the second part is still being computed.
       auto accumulate = [&](uint32_t c, auto&& between) {
-        const uint32_t stage = c & 1u;
+        const uint32_t s1 = c % kRing1;
         // dQ pass: the 16-bit dS of step c sits in the score buffer of step c (dead once the scores are read), so
         // the dP buffer is free for the next step as soon as the element-wise stage has read it
         const uint32_t col_u2 = kDKV ? kColT2 : ((c & 1u) ? kColT1b : kColT1);
-        const uint64_t b1n = kDescN | static_cast<uint64_t>((sm_b + stage * 2 * kTileBytes) >> 4);
-        const uint64_t b2n = kDescN | static_cast<uint64_t>((sm_b + stage * 2 * kTileBytes + kTileBytes) >> 4);
+        const uint64_t b1n = kDescN | static_cast<uint64_t>((sm_b1 + s1 * kTileBytes) >> 4);
         auto part = [&](int ks, uint32_t acc) {
-          const uint32_t ucol = (ks >> 2) * 64 + (ks & 3) * 8;
-          const uint64_t off = static_cast<uint64_t>((ks * 2048) >> 4);
-          if (kDKV) ptx::mma_ts(tmem + kColAcc1, tmem + kColT1 + ucol, b2n + off, idesc_acc1, acc);
-          ptx::mma_ts(tmem + kColAcc2, tmem + col_u2 + ucol, b1n + off, idesc_acc2, acc);
+          ptx::mma_ts(tmem + kColAcc2, tmem + col_u2 + (ks >> 2) * 64 + (ks & 3) * 8,
+                      b1n + static_cast<uint64_t>((ks * 2048) >> 4), idesc_acc2, acc);
         };
         w.wait(ptx::smem_u32(&bars->u_full[0]), c & 1u);
         ptx::tc_fence_after();
@@ -431,18 +460,43 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
         part(3, 1u);
         part(6, 1u);
         part(7, 1u);
-        ptx::mma_commit(ptx::smem_u32(&bars->b_free[stage]));
+        ptx::mma_commit(ptx::smem_u32(&bars->b1_free[s1]));
+        if (kDKV) ptx::mma_commit(ptx::smem_u32(&bars->b2_free[c % kRing2]));
+      };
+      auto accumulate_p = [&](uint32_t c) {
+        const uint32_t s2 = c % kRing2;
+        const uint64_t b2n = kDescN | static_cast<uint64_t>((sm_b2 + s2 * kTileBytes) >> 4);
+        auto part = [&](int ks, uint32_t acc) {
+          ptx::mma_ts(tmem + kColAcc1, tmem + kColT1 + (ks >> 2) * 64 + (ks & 3) * 8,
+                      b2n + static_cast<uint64_t>((ks * 2048) >> 4), idesc_acc1, acc);
+        };
+        w.wait(ptx::smem_u32(&bars->p_full[0]), c & 1u);
+        ptx::tc_fence_after();
+        part(0, c > first ? 1u : 0u);
+        part(1, 1u);
+        part(4, 1u);
+        part(5, 1u);
+        w.wait(ptx::smem_u32(&bars->p_full[1]), c & 1u);
+        ptx::tc_fence_after();
+        part(2, 1u);
+        part(3, 1u);
+        part(6, 1u);
+        part(7, 1u);
       };
       w.wait(ptx::smem_u32(&bars->a_full), tiles_done & 1u);
       for_each_step<kDKV>(p, s, tile0, head, [&](int, int, int) {
-        // dK/dV pass: the accumulate products of the last step must precede this step's T products (they overwrite
-        // U1 / U2).  dQ pass: only U2 is in use, T1 goes to its other buffer first.
-        if (kDKV && cnt > first) accumulate(cnt - 1, [] {});
-        const uint32_t stage = cnt & 1u;
-        w.wait(ptx::smem_u32(&bars->b_full[stage]), (cnt >> 1) & 1u);
+        // Products of one thread run in order, so one that overwrites a buffer may be issued right behind the one that read
+        // it.  dK/dV pass: dV of the last step (reads P in T1), the scores of this one (T1), dK of the last (dS in T2), dP
+        // of this one (T2) - the scores, on which most of the element-wise stage depends, do not wait for dS.  dQ pass: the
+        // scores go to T1's other buffer a step ahead of the dS, which takes the place of its scores.
+        if (kDKV && cnt > first) accumulate_p(cnt - 1);
+        const uint32_t s1 = cnt % kRing1, s2 = cnt % kRing2;
+        // (a poll costs this thread some 130 cycles: those of both tiles are in flight together)
+        const bool ok2 = ptx::mbar_try_wait(ptx::smem_u32(&bars->b2_full[s2]), (cnt / kRing2) & 1u);
+        w.wait(ptx::smem_u32(&bars->b1_full[s1]), (cnt / kRing1) & 1u);
         ptx::tc_fence_after();
-        const uint64_t b1 = kDescK | static_cast<uint64_t>((sm_b + stage * 2 * kTileBytes) >> 4);
-        const uint64_t b2 = kDescK | static_cast<uint64_t>((sm_b + stage * 2 * kTileBytes + kTileBytes) >> 4);
+        const uint64_t b1 = kDescK | static_cast<uint64_t>((sm_b1 + s1 * kTileBytes) >> 4);
+        const uint64_t b2 = kDescK | static_cast<uint64_t>((sm_b2 + s2 * kTileBytes) >> 4);
         const uint32_t col_t1 = (cnt & 1u) ? kColT1b : kColT1;
         auto product = [&](uint32_t col, uint64_t a, uint64_t b, bool half) {
           auto one = [&](int ks) {
@@ -457,16 +511,27 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
           }
         };
         product(tmem + col_t1, a1, b1, half1);
+        ptx::mma_commit(ptx::smem_u32(&bars->t1_full[cnt & 1u]));
         auto t2_product = [&]() {
+          if (!ok2) w.wait(ptx::smem_u32(&bars->b2_full[s2]), (cnt / kRing2) & 1u);
+          ptx::tc_fence_after();
           product(tmem + kColT2, a2, b2, half2);
-          ptx::mma_commit(ptx::smem_u32(&bars->t_full));
+          ptx::mma_commit(ptx::smem_u32(&bars->t2_full));
+          if (!kDKV) ptx::mma_commit(ptx::smem_u32(&bars->b2_free[s2]));
         };
         // dQ pass: first half of the last step's accumulate products, this step's dP product, then the second half
-        if (!kDKV && cnt > first) accumulate(cnt - 1, t2_product);
-        else t2_product();
+        if (!kDKV && cnt > first) {
+          accumulate(cnt - 1, t2_product);
+        } else {
+          if (cnt > first) accumulate(cnt - 1, [] {});
+          t2_product();
+        }
         ++cnt;
       });
-      if (cnt > first) accumulate(cnt - 1, [] {});
+      if (cnt > first) {
+        if (kDKV) accumulate_p(cnt - 1);
+        accumulate(cnt - 1, [] {});
+      }
       ptx::mma_commit(ptx::smem_u32(&bars->acc_full));
       w.wait(ptx::smem_u32(&bars->acc_full), tiles_done & 1u);   // all MMAs and their barrier arrivals are done before teardown
     }
@@ -516,25 +581,41 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
       ptx::mbar_arrive(ptx::smem_u32(&bars->bias_free));
     };
     for_each_step<kDKV>(p, s, tile0, head, [&](int, int srow0, int qh) {
-      w.wait(ptx::smem_u32(&bars->t_full), cnt & 1u);
-      ptx::tc_fence_after();
       // rows of the score tile are queries, columns keys - in the dK/dV pass the tile is held transposed
       const int q_first = kDKV ? srow0 : tile0, k_first = kDKV ? tile0 : srow0;
       const bool full = tile_is_full(s, q_first, kTileM, k_first, kTileN, p.mask_type, p.group) &&
                         (!kDKV || q_first + kTileM <= s.lq);
       const long long bias_bh = static_cast<long long>(b) * p.bias_bstride + static_cast<long long>(qh) * p.maxq * p.maxk;
-#pragma unroll 1
+      const uint32_t col_t1 = tmem + lane_base + ((cnt & 1u) ? kColT1b : kColT1) + 64 * grp;
+      const uint32_t col_t2 = tmem + lane_base + kColT2 + 64 * grp;
+      // bit e of bits[ch]: element (this row, column 64 grp + 32 ch + e) of the tile is visible
+      uint32_t bits[2];
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {
+        const int i0 = srow0 + 64 * grp + 32 * ch;
+        if (!kDKV) {
+          bits[ch] = !mine_ok ? 0u : (full ? 0xffffffffu : visible_bits(rb_mine, i0));
+        } else if (full) {
+          bits[ch] = 0xffffffffu;
+        } else if (mine >= s.lk) {
+          bits[ch] = 0u;
+        } else {
+          bits[ch] = (low_bits(hq_end - i0) & ~low_bits(c_lo - i0)) | low_bits(ctx_hi - i0) |
+                     (low_bits(t_hi - i0) & ~low_bits(t_lo - i0));
+        }
+      }
+      // Part one, as soon as the scores are there: P, and the factor f with dS = dP f, in the scores' registers.  The dP
+      // product runs meanwhile, and - dK/dV pass - dV and the next step's scores behind P.
+      uint32_t f[2][32];
+      w.wait(ptx::smem_u32(&bars->t1_full[cnt & 1u]), (cnt >> 1) & 1u);
+      ptx::tc_fence_after();
+      if (staged) w.wait(ptx::smem_u32(&bars->bias_full), cnt & 1u);
+#pragma unroll
       for (int ch = 0; ch < 2; ++ch) {
         const int col = 64 * grp + 32 * ch;
-        uint32_t t1[32], t2[32];
-        ptx::tmem_ld32(tmem + lane_base + ((cnt & 1u) ? kColT1b : kColT1) + col, t1);
-        ptx::tmem_ld32(tmem + lane_base + kColT2 + col, t2);
-        // dK/dV pass: this key's bias values for the 32 queries of the chunk lie a row pitch apart - all 32 loads
-        // are issued here, ahead of the wait for the products (addresses clamped into the plane: what lies outside
-        // the sequence is never used)
-        uint32_t bcol[16];
+        ptx::tmem_ld32(col_t1 + 32 * ch, f[ch]);
+        uint32_t bcol[16];   // the bias values of the 32 elements, packed
         if (staged && !kDKV) {
-          if (ch == 0) w.wait(ptx::smem_u32(&bars->bias_full), cnt & 1u);
           // this query's 32 keys col .. col + 31: box col / 64 (= grp), row = query, four 16-byte chunks from
           // (col % 64) / 8 on, each ^ (query & 7)
           const uint32_t rowbase = sm_bias + grp * (kTileM * 128) + row * 128;
@@ -546,9 +627,6 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
                          : "r"(rowbase + (((c16 + q4) ^ (row & 7)) << 4)));
           if (ch == 1) release_bias();   // this thread has read its row
         } else if (staged) {
-          if (ch == 0) {
-            w.wait(ptx::smem_u32(&bars->bias_full), cnt & 1u);
-          }
           // element (query col + e, key row): box row / 64, row = query, 16-byte chunk (key % 64) / 8 ^ (query & 7)
           const uint32_t box = sm_bias + (row >> 6) * (kTileM * 128) + (row & 7) * 2;
           const uint32_t kchunk = (row & 63) >> 3;
@@ -562,6 +640,8 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
           }
           if (ch == 1) release_bias();   // this thread has read its column
         } else if (kDKV && p.bias) {
+          // this key's bias values for the 32 queries lie a row pitch apart (addresses clamped into the plane: what lies
+          // outside the sequence is never used)
           const int kk = mine < p.maxk ? mine : p.maxk - 1;
           const unsigned short* bsrc = static_cast<const unsigned short*>(p.bias) + bias_bh + kk;
 #pragma unroll
@@ -571,84 +651,77 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
             const uint32_t hi = __ldg(bsrc + static_cast<long long>(r1 < p.maxq ? r1 : p.maxq - 1) * p.maxk);
             bcol[e] = lo | (hi << 16);
           }
-        }
-        ptx::tmem_wait_ld();
-        // bit e of `bits`: element (this row, column col + e) of the tile is visible
-        uint32_t bits;
-        if (!kDKV) {
-          bits = !mine_ok ? 0u : (full ? 0xffffffffu : visible_bits(rb_mine, srow0 + col));
-        } else if (full) {
-          bits = 0xffffffffu;
-        } else if (mine >= s.lk) {
-          bits = 0u;
-        } else {
-          const int i0 = srow0 + col;
-          bits = (low_bits(hq_end - i0) & ~low_bits(c_lo - i0)) | low_bits(ctx_hi - i0) |
-                 (low_bits(t_hi - i0) & ~low_bits(t_lo - i0));
-        }
-        uint32_t u1[16], u2[16];
-        // per warp: every element visible -> no selects; nothing visible -> zeros without arithmetic; else selects
-        const bool all_on = __all_sync(0xffffffffu, bits == 0xffffffffu);
-        const bool all_off = __all_sync(0xffffffffu, bits == 0u);
-        if (all_off) {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) u1[e] = u2[e] = 0u;
-        } else if (staged && !kDKV) {
-          // (values of rows / keys outside the sequence are never used: their elements are not visible)
-#pragma unroll
-          for (int e = 0; e < 16; ++e)
-            score_grad2<T, true, true>(make_float2(__uint_as_float(t1[2 * e]), __uint_as_float(t1[2 * e + 1])),
-                                       make_float2(__uint_as_float(t2[2 * e]), __uint_as_float(t2[2 * e + 1])),
-                                       BPack<T>::unpack(bcol[e]), p.alpha, p.scale, (bits >> (2 * e)) & 3u, u1[e], u2[e]);
-        } else if (!kDKV && bias_vec && mine_ok && srow0 + col + 32 <= p.maxk) {
-          // dQ pass: the 32 bias values of this row and chunk are contiguous - four 16-byte loads
-          const uint4* src = reinterpret_cast<const uint4*>(static_cast<const T*>(p.bias) + bias_bh +
-                                                            static_cast<long long>(mine) * p.maxk + srow0 + col);
-          uint32_t bw[16];
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            const uint4 v4 = __ldg(src + q4);
-            bw[4 * q4] = v4.x, bw[4 * q4 + 1] = v4.y, bw[4 * q4 + 2] = v4.z, bw[4 * q4 + 3] = v4.w;
-          }
-#pragma unroll
-          for (int e = 0; e < 16; ++e)
-            score_grad2<T, true, true>(make_float2(__uint_as_float(t1[2 * e]), __uint_as_float(t1[2 * e + 1])),
-                                       make_float2(__uint_as_float(t2[2 * e]), __uint_as_float(t2[2 * e + 1])),
-                                       BPack<T>::unpack(bw[e]), p.alpha, p.scale, (bits >> (2 * e)) & 3u, u1[e], u2[e]);
         } else if (p.bias) {
+          const long long at = bias_bh + static_cast<long long>(mine) * p.maxk + srow0 + col;
+          if (bias_vec && mine_ok && srow0 + col + 32 <= p.maxk) {   // contiguous: four 16-byte loads
+            const uint4* src = reinterpret_cast<const uint4*>(static_cast<const T*>(p.bias) + at);
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {
+              const uint4 v4 = __ldg(src + q4);
+              bcol[4 * q4] = v4.x, bcol[4 * q4 + 1] = v4.y, bcol[4 * q4 + 2] = v4.z, bcol[4 * q4 + 3] = v4.w;
+            }
+          } else {
+            const unsigned short* src = static_cast<const unsigned short*>(p.bias) + at;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const uint32_t v2 = (bits[ch] >> (2 * e)) & 3u;
+              const uint32_t lo = (v2 & 1u) ? src[2 * e] : 0u, hi = (v2 & 2u) ? src[2 * e + 1] : 0u;
+              bcol[e] = lo | (hi << 16);
+            }
+          }
+        }
+        ptx::tmem_wait_ld_dep(f[ch]);
+        // per warp: every element visible -> no selects; nothing visible -> zeros without arithmetic; else selects
+        uint32_t u1[16];
+        auto compute = [&](auto bias_on, auto select) {
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const uint32_t v2 = (bits >> (2 * e)) & 3u;
-            const int c = col + 2 * e;
-            float2 bias;
-            if (kDKV) {
-              const float2 both = BPack<T>::unpack(bcol[e]);
-              bias.x = (v2 & 1u) ? both.x : 0.f;
-              bias.y = (v2 & 2u) ? both.y : 0.f;
-            } else {
-              const long long at = bias_bh + static_cast<long long>(mine) * p.maxk + srow0 + c;
-              bias.x = (v2 & 1u) ? BPack<T>::one(p.bias, at) : 0.f;
-              bias.y = (v2 & 2u) ? BPack<T>::one(p.bias, at + 1) : 0.f;
-            }
-            score_grad2<T, true, true>(make_float2(__uint_as_float(t1[2 * e]), __uint_as_float(t1[2 * e + 1])),
-                                       make_float2(__uint_as_float(t2[2 * e]), __uint_as_float(t2[2 * e + 1])), bias,
-                                       p.alpha, p.scale, v2, u1[e], u2[e]);
+            const float2 v = score_part<T, decltype(bias_on)::value, decltype(select)::value>(
+                make_float2(__uint_as_float(f[ch][2 * e]), __uint_as_float(f[ch][2 * e + 1])),
+                decltype(bias_on)::value ? BPack<T>::unpack(bcol[e]) : make_float2(0.f, 0.f), p.alpha, p.scale,
+                (bits[ch] >> (2 * e)) & 3u, u1[e]);
+            f[ch][2 * e] = __float_as_uint(v.x);
+            f[ch][2 * e + 1] = __float_as_uint(v.y);
           }
-        } else if (all_on) {
+        };
+        if (__all_sync(0xffffffffu, bits[ch] == 0u)) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e)
-            score_grad2<T, false, false>(make_float2(__uint_as_float(t1[2 * e]), __uint_as_float(t1[2 * e + 1])),
-                                         make_float2(__uint_as_float(t2[2 * e]), __uint_as_float(t2[2 * e + 1])),
-                                         make_float2(0.f, 0.f), p.alpha, p.scale, 3u, u1[e], u2[e]);
+          for (int e = 0; e < 16; ++e) u1[e] = 0u;
+        } else if (staged || p.bias) {
+          compute(std::true_type{}, std::true_type{});
+        } else if (__all_sync(0xffffffffu, bits[ch] == 0xffffffffu)) {
+          compute(std::false_type{}, std::false_type{});
+        } else {
+          compute(std::false_type{}, std::true_type{});
+        }
+        if (kDKV) {
+          ptx::tmem_st16(col_t1 + 16 * ch, u1);
+          ptx::tmem_wait_st();
+          ptx::tc_fence_before();
+          ptx::mbar_arrive(ptx::smem_u32(&bars->p_full[ch]));
+        }
+      }
+      // Part two: dS = dP f
+      w.wait(ptx::smem_u32(&bars->t2_full), cnt & 1u);
+      ptx::tc_fence_after();
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {
+        const int col = 64 * grp + 32 * ch;
+        uint32_t t2[32], u2[16];
+        ptx::tmem_ld32(col_t2 + 32 * ch, t2);
+        ptx::tmem_wait_ld_dep(t2);
+        if (__all_sync(0xffffffffu, bits[ch] == 0u)) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) u2[e] = 0u;
         } else {
 #pragma unroll
-          for (int e = 0; e < 16; ++e)
-            score_grad2<T, false, true>(make_float2(__uint_as_float(t1[2 * e]), __uint_as_float(t1[2 * e + 1])),
-                                        make_float2(__uint_as_float(t2[2 * e]), __uint_as_float(t2[2 * e + 1])),
-                                        make_float2(0.f, 0.f), p.alpha, p.scale, (bits >> (2 * e)) & 3u, u1[e], u2[e]);
+          for (int e = 0; e < 16; ++e) {
+            const float2 ds = __fmul2_rn(make_float2(__uint_as_float(t2[2 * e]), __uint_as_float(t2[2 * e + 1])),
+                                         make_float2(__uint_as_float(f[ch][2 * e]), __uint_as_float(f[ch][2 * e + 1])));
+            u2[e] = BPack<T>::pack((bits[ch] >> (2 * e)) & 1u ? ds.x : 0.f, (bits[ch] >> (2 * e)) & 2u ? ds.y : 0.f);
+          }
         }
-        if (kDKV) ptx::tmem_st16(tmem + lane_base + kColT1 + 64 * grp + 16 * ch, u1);
-        ptx::tmem_st16(tmem + lane_base + (kDKV ? kColT2 : ((cnt & 1u) ? kColT1b : kColT1)) + 64 * grp + 16 * ch, u2);
+        ptx::tmem_st16((kDKV ? col_t2 : col_t1) + 16 * ch, u2);
         ptx::tmem_wait_st();
         ptx::tc_fence_before();
         ptx::mbar_arrive(ptx::smem_u32(&bars->u_full[ch]));
@@ -737,10 +810,6 @@ cudaError_t launch_bwd_tc_t(const BwdParams& bp, int dtype, int num_sms, cudaStr
       !make_tile_map(&mg, bp.dout, p.total_q, p.hq, p.dv, dtype) ||
       !make_tile_map(&mk, p.k, p.total_k, p.hk, p.dqk, dtype) || !make_tile_map(&mv, p.v, p.total_k, p.hk, p.dv, dtype))
     return cudaErrorNotSupported;
-  constexpr int smem = 1024 + 6 * (D / 64) * kTileM * 128 + 256;
-  constexpr int smem_kv = smem + 2 * kTileM * 128;   // + the staged bias tile of the dK/dV pass
-  static_assert(smem_kv <= 232448, "shared memory budget of one CTA exceeded");
-  static_assert(sizeof(BwdBars) <= 256, "barrier block too large");
   // the bias as TMA tiles: rows 16-byte aligned and batch blocks back to back (what the forward's staged mode needs)
   CUtensorMap mb = mq;
   const int bias_staged = p.bias && (p.maxk % 8 == 0) && (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0 &&
@@ -770,7 +839,7 @@ cudaError_t launch_bwd_tc_t(const BwdParams& bp, int dtype, int num_sms, cudaStr
       cfg.numAttrs = (!kDKV || overlap) ? 1 : 0;
       return cudaLaunchKernelEx(&cfg, kern, bp, a1, a2, b1, b2, mb);
     };
-    return bias_staged ? go(hstu_bwd_tc_kernel<D, T, kDKV, true>, smem_kv) : go(hstu_bwd_tc_kernel<D, T, kDKV, false>, smem);
+    return bias_staged ? go(hstu_bwd_tc_kernel<D, T, kDKV, true>, BwdRings<D, true, kDKV>::kSmem) : go(hstu_bwd_tc_kernel<D, T, kDKV, false>, BwdRings<D, false, kDKV>::kSmem);
   };
   cudaError_t e = cudaSuccess;
   overlap = p.total_q > 0;   // (a dQ pass is launched in front of the dK/dV pass)
