@@ -451,7 +451,7 @@ cudaError_t launch_simt_bwd(const BwdParams& bp, cudaStream_t stream) {
 }
 
 // The register-tiled kernels wherever their loads are possible.  (16 sequences of 50-500 rows, 2 heads of 64, fp32, forward
-// and backward: 169 us, 1236 us with the other kernels.)
+// and backward: 158 us, 1239 us with the other kernels.)
 bool simt_bwd_supported(const BwdParams& bp, int dtype) {
   return simt::dims_ok(bp.f) && simt::aligned_to(bp.f.q, dtype) && simt::aligned_to(bp.f.k, dtype) &&
          simt::aligned_to(bp.f.v, dtype) && simt::aligned_to(bp.dout, dtype) && simt::aligned_to(bp.dq, dtype) &&
