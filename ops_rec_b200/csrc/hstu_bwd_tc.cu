@@ -48,6 +48,7 @@ constexpr long long kBwdWaitLimit = 2000000000ll;  // ~1 s of SM clock
 template <typename T> struct BPack;
 template <> struct BPack<__nv_bfloat16> {
   static constexpr int kFormat = 1;
+  static constexpr bool kExact = false;   // sigmoid: the tanh form
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -59,8 +60,12 @@ template <> struct BPack<__nv_bfloat16> {
     return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
   }
 };
+template <> struct BPack<Bf16Exp> : BPack<__nv_bfloat16> {
+  static constexpr bool kExact = true;    // sigmoid: exp2 and reciprocal
+};
 template <> struct BPack<__half> {
   static constexpr int kFormat = 0;
+  static constexpr bool kExact = true;
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -147,7 +152,7 @@ template <typename T, bool kBiasOn, bool kSelect>
 __device__ __forceinline__ float2 score_part(float2 s, float2 bias, float alpha, float scale, uint32_t vis, uint32_t& p_out) {
   if (kBiasOn) s = __fadd2_rn(s, bias);
   float2 pv, f;
-  if (BPack<T>::kFormat == 0) {   // fp16: exp2 and reciprocal
+  if (BPack<T>::kExact) {
     const float2 x = __fmul2_rn(s, make_float2(alpha, alpha));
     const float2 ny = __fmul2_rn(x, make_float2(-1.4426950408889634f, -1.4426950408889634f));
     const float2 d = __fadd2_rn(make_float2(ptx::ex2_approx(ny.x), ptx::ex2_approx(ny.y)), make_float2(1.f, 1.f));
@@ -883,6 +888,9 @@ bool bwd_tc_supported(const BwdParams& bp, int dtype) {
 cudaError_t launch_bwd_tc(const BwdParams& bp, int dtype, int num_sms, cudaStream_t stream) {
   const KParams& p = bp.f;
   const bool wide = p.dqk > 64 || p.dv > 64;
+  if (dtype == HSTU_DTYPE_BF16 && !tanh_silu(p))   // (the forward's rule)
+    return wide ? launch_bwd_tc_t<128, Bf16Exp>(bp, dtype, num_sms, stream)
+                : launch_bwd_tc_t<64, Bf16Exp>(bp, dtype, num_sms, stream);
   if (dtype == HSTU_DTYPE_BF16)
     return wide ? launch_bwd_tc_t<128, __nv_bfloat16>(bp, dtype, num_sms, stream)
                         : launch_bwd_tc_t<64, __nv_bfloat16>(bp, dtype, num_sms, stream);

@@ -6,6 +6,7 @@
 // classifier (ascendc/attention/hstu_v1/hstu_forward_v1/op_kernel/atlas950/hstu_dense_causal_mask.h:63-109).
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -153,6 +154,18 @@ HSTU_HD SeqInfo make_seq(const KParams& p, const SeqRaw& r) {
   return s;
 }
 HSTU_HD SeqInfo load_seq(const KParams& p, int b) { return make_seq(p, read_seq(p, b)); }
+
+// The element type of a bf16 call whose SiLU is formed from exp2 and a reciprocal, as fp16's is, instead of tanh.approx.
+// P = x (1 + tanh(x/2)) / 2 from tanh.approx is right to its rounding to bf16 for x > -6, but 0.5 % off at x = -8 and 1 %
+// at -12 (the exp2 form: 0.3 %, the rounding).  Only the head dims the tensor-core kernels are tuned for, 64 and 128, take
+// it (one SFU operation per score instead of two); every other pair of dims keeps 32-bit accuracy up to the rounding of P.
+struct Bf16Exp {
+  __nv_bfloat16 v;
+  Bf16Exp() = default;
+  explicit __device__ __forceinline__ Bf16Exp(float x) : v(__float2bfloat16_rn(x)) {}
+};
+static_assert(sizeof(Bf16Exp) == 2 && alignof(Bf16Exp) == 2, "layout of a bf16 value");
+inline bool tanh_silu(const KParams& p) { return p.dqk == p.dv && (p.dqk == 64 || p.dqk == 128); }
 
 // Input consistency of one sequence (HSTU_ST_* bits).  The reference does not check these and would read
 // out of bounds (the bias/mask row stride is max_seq_len_k).

@@ -428,8 +428,8 @@ hstu_short_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, con
     // ------------------------------------------------------------------ P / O (thread = row)
     const int row = threadIdx.x;
     const uint32_t t_s = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-    constexpr bool kExact = Pack<T>::kFormat == 0;
-    const float c_in = kExact ? p.alpha : 0.5f * p.alpha;   // (bf16: the tanh form, on half the argument)
+    constexpr bool kExact = Pack<T>::kExact;
+    const float c_in = kExact ? p.alpha : 0.5f * p.alpha;   // (the tanh form: on half the argument)
     auto arrive_warp = [&](uint64_t* bar) {
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(bar));
@@ -618,6 +618,10 @@ cudaError_t launch_short(const KParams& p, int dtype, const CUtensorMap& mq, con
                 : launch_inst<DD, TT, false>(p, mq, mk, mv, mbs, mc, num_sms, stream)
   const bool wide = p.dqk > 64 || p.dv > 64;
   if (dtype == HSTU_DTYPE_BF16) {
+    if (!tanh_silu(p)) {
+      if (wide) { HSTU_SHORT_CASE(128, Bf16Exp); }
+      HSTU_SHORT_CASE(64, Bf16Exp);
+    }
     if (wide) { HSTU_SHORT_CASE(128, __nv_bfloat16); }
     HSTU_SHORT_CASE(64, __nv_bfloat16);
   }

@@ -708,8 +708,8 @@ hstu_tc_kernel(const KParams p, const __grid_constant__ CUtensorMap tm_q, const 
     const int row = (threadIdx.x - 128) & 127;  // row inside a tile == TMEM lane
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const bool alpha_first = (p.flags & HSTU_FLAG_ALPHA_BEFORE_BIAS) != 0;
-    constexpr bool kExact = Pack<T>::kFormat == 0;
-    // bf16 works on a = y / 2 (tanh form), fp16 on y itself;  x = c_in * s + c_bias * bias
+    constexpr bool kExact = Pack<T>::kExact;
+    // the tanh form works on a = y / 2, the exp2 form on y itself;  x = c_in * s + c_bias * bias
     const float c_in = kExact ? p.alpha : 0.5f * p.alpha;
     const float c_bias = alpha_first ? (kExact ? 1.f : 0.5f) : c_in;
     // (per Q tile, as scalars: the loop over the two tiles is not unrolled - this role's code is what the SM's
@@ -1107,6 +1107,10 @@ cudaError_t launch_tc(const KParams& p_in, int dtype, int num_sms, cudaStream_t 
                           : launch_inst<DD, TT, 0, false>(p, mq, mk, mv, mb, mo, mc, vec_ok, g, stream)
   const bool wide = p.dqk > 64 || p.dv > 64;
   if (dtype == HSTU_DTYPE_BF16) {
+    if (!tanh_silu(p)) {
+      if (wide) { HSTU_TC_CASE(128, Bf16Exp); }
+      HSTU_TC_CASE(64, Bf16Exp);
+    }
     if (wide) { HSTU_TC_CASE(128, __nv_bfloat16); }
     HSTU_TC_CASE(64, __nv_bfloat16);
   }

@@ -49,6 +49,7 @@ struct Waiter {
 template <typename T> struct Pack;
 template <> struct Pack<__nv_bfloat16> {
   static constexpr int kFormat = 1;
+  static constexpr bool kExact = false;   // SiLU: the tanh form
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -60,8 +61,12 @@ template <> struct Pack<__nv_bfloat16> {
     return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
   }
 };
+template <> struct Pack<Bf16Exp> : Pack<__nv_bfloat16> {
+  static constexpr bool kExact = true;    // SiLU: exp2 and reciprocal
+};
 template <> struct Pack<__half> {
   static constexpr int kFormat = 0;
+  static constexpr bool kExact = true;
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -83,7 +88,7 @@ template <> struct Pack<__half> {
 template <typename T, int kBias, bool kMasked>
 __device__ __forceinline__ void silu_chunk(const uint32_t (&sr)[32], const uint32_t (&bv)[16], uint32_t (&pr)[16],
                                            float c_in, float c_bias, float scale, uint32_t visible) {
-  constexpr bool kExact = Pack<T>::kFormat == 0;  // fp16: exp2 + rcp (two MUFU ops); bf16: tanh form (one)
+  constexpr bool kExact = Pack<T>::kExact;  // exp2 + rcp (two MUFU ops); else the tanh form (one)
   const float2 cin2 = make_float2(c_in, c_in);
   const float2 cb2 = make_float2(c_bias, c_bias);
   const float2 sc2 = make_float2(scale, scale);
