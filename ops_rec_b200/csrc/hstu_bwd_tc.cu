@@ -439,6 +439,8 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
       constexpr uint64_t kDescN = ptx::umma_desc_sw128_hi(kHalfBytes, 1024);   // the same tiles read N-major
       const uint64_t a1 = kDescK | static_cast<uint64_t>(sm_a >> 4);
       const uint64_t a2 = kDescK | static_cast<uint64_t>((sm_a + kTileBytes) >> 4);
+      // Whether the upper 64 rows of the last step's streamed tile hold any of the sequence: else their products are left out.
+      bool upper = true;
       // Accumulate products of step c: Acc1 += P.B2 (dK/dV pass), Acc2 += dS.B1.  The element-wise groups hand P and dS over
       // in two parts each (values 0..31 and 64..95 of a tile row, then the rest), so the first half of these MMAs runs
       // while the second part is still being computed.
@@ -456,15 +458,19 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
         ptx::tc_fence_after();
         part(0, c > first ? 1u : 0u);
         part(1, 1u);
-        part(4, 1u);
-        part(5, 1u);
+        if (upper) {
+          part(4, 1u);
+          part(5, 1u);
+        }
         w.wait(ptx::smem_u32(&bars->u_full[1]), c & 1u);
         ptx::tc_fence_after();
         between();   // (dQ pass: the dP product of the next step - its buffer has been read completely by now)
         part(2, 1u);
         part(3, 1u);
-        part(6, 1u);
-        part(7, 1u);
+        if (upper) {
+          part(6, 1u);
+          part(7, 1u);
+        }
         ptx::mma_commit(ptx::smem_u32(&bars->b1_free[s1]));
         if (kDKV) ptx::mma_commit(ptx::smem_u32(&bars->b2_free[c % kRing2]));
       };
@@ -479,17 +485,21 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
         ptx::tc_fence_after();
         part(0, c > first ? 1u : 0u);
         part(1, 1u);
-        part(4, 1u);
-        part(5, 1u);
+        if (upper) {
+          part(4, 1u);
+          part(5, 1u);
+        }
         w.wait(ptx::smem_u32(&bars->p_full[1]), c & 1u);
         ptx::tc_fence_after();
         part(2, 1u);
         part(3, 1u);
-        part(6, 1u);
-        part(7, 1u);
+        if (upper) {
+          part(6, 1u);
+          part(7, 1u);
+        }
       };
       w.wait(ptx::smem_u32(&bars->a_full), tiles_done & 1u);
-      for_each_step<kDKV>(p, s, tile0, head, [&](int, int, int) {
+      for_each_step<kDKV>(p, s, tile0, head, [&](int, int srow0, int) {
         // Products of one thread run in order, so one that overwrites a buffer may be issued right behind the one that read
         // it.  dK/dV pass: dV of the last step (reads P in T1), the scores of this one (T1), dK of the last (dS in T2), dP
         // of this one (T2) - the scores, on which most of the element-wise stage depends, do not wait for dS.  dQ pass: the
@@ -531,6 +541,7 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
           if (cnt > first) accumulate(cnt - 1, [] {});
           t2_product();
         }
+        upper = (kDKV ? s.lq : s.lk) - srow0 > 64;
         ++cnt;
       });
       if (cnt > first) {
@@ -614,6 +625,23 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
       uint32_t f[2][32];
       w.wait(ptx::smem_u32(&bars->t1_full[cnt & 1u]), (cnt >> 1) & 1u);
       ptx::tc_fence_after();
+      // The last streamed tile of a sequence holds foreign rows behind the sequence's end.  P and dS are 0 there, but 0 x NaN is
+      // not: the rows up to the next multiple of 64 (the accumulate products stop there) are zeroed before the results that
+      // meet them are handed over (B1: dS; in the dK/dV pass B2: P).  The scores have read B1 by now; what the dP product
+      // still reads of B2 belongs to masked elements.  (Forward and backward of 64 sequences of mean 2400 4537 -> 4596 us,
+      // 32 of 256-1024 162 -> 165, 1024 of 20-300 646 -> 677.  In the two idle warps, with the products waiting for it, it
+      // cost more: 4599 / 169 / 752.  A multiple of 16 with a predicate on every product: 4585 / 164 / 684.)
+      const int rem = (kDKV ? s.lq : s.lk) - srow0;
+      if (rem < kTileM && (rem & 63)) {
+        const bool second = kDKV && grp == 1;
+        const uint32_t s1 = cnt % kRing1, s2 = cnt % kRing2;
+        if (second) w.wait(ptx::smem_u32(&bars->b2_full[s2]), (cnt / kRing2) & 1u);
+        const uint32_t first_row = (second ? sm_b2 + s2 * kTileBytes : sm_b1 + s1 * kTileBytes) + rem * 128;
+        const int boxes = second ? halves2 : halves1;
+        for (int i = kDKV ? row : tid - 128; i < (64 - (rem & 63)) * 8; i += kDKV ? kTileM : 2 * kTileM)
+          for (int hf = 0; hf < boxes; ++hf) ptx::st_shared_zero16(first_row + hf * kHalfBytes + i * 16);
+        ptx::fence_proxy_async();
+      }
       if (staged) w.wait(ptx::smem_u32(&bars->bias_full), cnt & 1u);
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {

@@ -408,3 +408,33 @@ def test_head_dims_narrower_than_a_tile(Dqk, Dv, dtype, bias, tgt):
     got, status = run_bwd(grad, args)
     assert status == 0
     assert_bwd_parity(got, grad, args, label=f"{Dqk}x{Dv} {dtype}")
+
+
+@pytest.mark.parametrize("poison", [float("nan"), float("inf")])
+@pytest.mark.parametrize("Dqk,Dv,dtype", [(64, 64, BF16), (128, 128, BF16), (32, 32, FP16), (64, 128, BF16), (128, 64, FP16),
+                                          (8, 16, BF16)])
+@pytest.mark.parametrize("extra", [dict(bias=False), dict(bias=True, tgt=5, g=2), dict(bias=False, delta=True)])
+def test_non_finite_values_of_a_neighbouring_sequence_do_not_leak(Dqk, Dv, dtype, extra, poison):
+    """The streamed tiles run past a sequence's end into the next sequence's rows, or into rows behind the last offset: with
+    every second sequence and those rows non-finite, the other sequences' gradients are bit for bit what they are without."""
+    grad, args = make_bwd_case(9, 4, 2, Dqk, Dv, 300, dtype, seed=Dqk + Dv, alpha=1.0 / Dqk, **extra)
+    pad = lambda t, value: torch.cat([t, torch.full((130, *t.shape[1:]), value, dtype=t.dtype)])
+    tensors = dict(q=args["q"], k=args["k"], v=args["v"], grad=grad)
+    offs = {n: (args["seq_offset_k"] if n in "kv" else args["seq_offset"]).tolist() for n in tensors}
+    res = []
+    for value in (0.0, poison):
+        t = {n: pad(x, value) for n, x in tensors.items()}
+        for b in range(1, 9, 2):
+            for n, x in t.items():
+                if value:
+                    x[offs[n][b]:offs[n][b + 1]] = value
+        got, status = run_bwd(t["grad"], dict(args, q=t["q"], k=t["k"], v=t["v"]))
+        assert status == 0
+        res.append(got)
+    for b in range(0, 9, 2):
+        for i, n in enumerate(("q", "k", "v")):
+            rows = slice(offs[n][b], offs[n][b + 1])
+            assert torch.isfinite(res[1][i][rows].float()).all(), (NAMES[i], b)
+            assert torch.equal(res[0][i][rows], res[1][i][rows]), (NAMES[i], b)
+        if args["attn_bias"] is not None:
+            assert torch.equal(res[0][3][b], res[1][3][b]), b
