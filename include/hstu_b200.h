@@ -285,9 +285,8 @@ HSTU_API int ops_rec_in_linear_silu_bwd(const OpsRecInLinearSiluBwdArgs* args, v
  * (0 = inputs were consistent).  The reference reads out of bounds on such inputs without noticing. */
 HSTU_API int hstu_jagged_fwd_status(const void* workspace, void* stream, uint32_t* status);
 
-/* Which kernel phase 2 would run for these arguments: 1 = tcgen05 tensor-core kernel at its own tile width (dim_qk =
- * dim_v = 64 or 128), 0 = anything else (the generic kernel, or the tensor-core kernel with tiles wider than the head
- * dims), negative = error code. */
+/* Which kernel phase 2 would run for these arguments: 1 = a tcgen05 tensor-core kernel, 0 = a CUDA-core kernel,
+ * negative = error code. */
 HSTU_API int hstu_jagged_fwd_kernel_kind(const HstuJaggedArgs* args);
 
 /* Host-side run of the scheduling pre-pass on HOST copies of the offsets (the same ordering rule the device

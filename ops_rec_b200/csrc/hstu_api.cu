@@ -19,6 +19,7 @@ cudaError_t launch_bwd_prepass(const KParams& p, cudaStream_t stream);
 long long plan_host(const KParams& p, uint32_t* items, long long capacity, uint32_t* status);
 bool tc_supported(const KParams& p, int dtype);
 bool short_paged_split(const KParams& p);
+bool tc_runs_short(const KParams& p);
 cudaError_t launch_tc(const KParams& p, int dtype, int num_sms, cudaStream_t stream);
 cudaError_t launch_bwd_generic(const BwdParams& bp, int dtype, cudaStream_t stream);
 bool bwd_tc_supported(const BwdParams& bp, int dtype);
@@ -191,7 +192,7 @@ int hstu_jagged_fwd_kernel_kind(const HstuJaggedArgs* args) {
   int rc = validate(args);
   if (rc) return rc;
   const hstu::KParams p = to_params(args, nullptr, 0);
-  return wants_tc(args, p) && args->dim_qk == args->dim_v && args->dim_qk % 64 == 0 ? 1 : 0;
+  return wants_tc(args, p) ? 1 : 0;
 }
 
 // `paged` (hstu_paged only): parameters that carry the page table, for the pre-pass's consistency check.
@@ -654,6 +655,11 @@ int hstu_debug_mask_host(int32_t len_q, int32_t len_k, int32_t num_context, int3
 
 // For the q-tile of rows [r0, r0 + rows): number of K tiles of width bn to visit, and (bit t of full_bits,
 // t < 64) whether K tile t is classified "no predicate needed".
+int hstu_debug_short_form(const HstuJaggedArgs* args) {
+  const int kind = hstu_jagged_fwd_kernel_kind(args);
+  return kind == 1 ? (hstu::tc_runs_short(to_params(args, nullptr, 0)) ? 1 : 0) : kind;
+}
+
 int hstu_debug_tiles_host(int32_t len_q, int32_t len_k, int32_t num_context, int32_t num_target,
                           int32_t target_group_size, int32_t mask_type, int32_t r0, int32_t rows, int32_t bn,
                           uint64_t* full_bits) {

@@ -58,10 +58,11 @@ HSTU_API int hstu_jagged_fwd_static(const HstuJaggedArgs* args, void* stream) {
   uint64_t need = 0;
   int rc = hstu_jagged_fwd_get_workspace_size(args, &need);  // validates args; host arithmetic only
   if (rc) return rc;
-  // (head dims that are not a tile width of the tensor-core kernel: the generic kernel needs no list, so it takes the
-  // batches whose list is too long)
+  // The CUDA-core kernels need no list.  Where one is too long they take the calls whose head dims are not 64 or 128 - such a
+  // call then runs, slower, rather than not at all.  (At 64 and 128 the refusal below stays: callers fall back on it.)
   HstuJaggedArgs listless = *args;
-  if (need > HSTU_STATIC_SCRATCH_BYTES && hstu_jagged_fwd_kernel_kind(args) == 0) {
+  const bool tile_width = args->dim_qk == args->dim_v && (args->dim_qk == 64 || args->dim_qk == 128);
+  if (need > HSTU_STATIC_SCRATCH_BYTES && !tile_width) {
     listless.flags |= HSTU_FLAG_FORCE_GENERIC;
     args = &listless;
     rc = hstu_jagged_fwd_get_workspace_size(args, &need);

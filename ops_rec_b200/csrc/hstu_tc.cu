@@ -1060,6 +1060,26 @@ bool tc_supported(const KParams& p, int dtype) {
   return (align & 15u) == 0;
 }
 
+// 16-byte loads of bias (or custom mask) rows are possible.
+static bool bias_rows_aligned(const KParams& p) {
+  return p.bias && (p.maxk % 8 == 0) && (p.bias_bstride % 8 == 0) && (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0;
+}
+// How the bias reaches the scores: 0 there is none, 1 plain loads, 2 tiles staged by TMA, 3 a custom mask (in the bias's
+// operand slot).  Staging needs 16-byte aligned rows and batch blocks laid out back to back (or one shared block); the
+// tensor cores then add the tile to S, which gives alpha * (S + bias) only.
+static int bias_mode_of(const KParams& p) {
+  if (p.mask_type == HSTU_MASK_CUSTOM) return 3;
+  if (!p.bias) return 0;
+  const bool staged = bias_rows_aligned(p) && !(p.flags & HSTU_FLAG_ALPHA_BEFORE_BIAS) &&
+                      (p.bias_bstride == 0 || p.bias_bstride == static_cast<long long>(p.hq) * p.maxq * p.maxk);
+  return staged ? 2 : 1;
+}
+// Whether a call this file supports goes to the kernel for short sequences.
+bool tc_runs_short(const KParams& p) {
+  const int mode = bias_mode_of(p);
+  return (mode == 0 || mode == 2) && short_preferred(p);
+}
+
 // Returns cudaSuccess, a CUDA error, or cudaErrorNotSupported when the tensor maps could not be encoded.
 cudaError_t launch_tc(const KParams& p_in, int dtype, int num_sms, cudaStream_t stream) {
   KParams p = p_in;
@@ -1075,17 +1095,10 @@ cudaError_t launch_tc(const KParams& p_in, int dtype, int num_sms, cudaStream_t 
   long long grid = p.item_capacity < num_sms ? p.item_capacity : num_sms;
   if (grid < 1) grid = 1;
   const int g = static_cast<int>(grid);
-  const int vec_ok = p.bias && (p.maxk % 8 == 0) && (p.bias_bstride % 8 == 0) &&
-                     (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0;
-  // bias staging by TMA needs 16-byte aligned rows and batch blocks laid out back to back (or one shared block);
-  // the tensor cores then add the tile to S, which gives alpha * (S + bias) only
-  int bias_mode = p.bias ? 1 : 0;
+  const int vec_ok = bias_rows_aligned(p);
+  int bias_mode = bias_mode_of(p);
   CUtensorMap mb = mq;
-  if (custom_mask) bias_mode = 3;
-  if (!custom_mask && p.bias && vec_ok && !(p.flags & HSTU_FLAG_ALPHA_BEFORE_BIAS) &&
-      (p.bias_bstride == 0 || p.bias_bstride == static_cast<long long>(p.hq) * p.maxq * p.maxk) &&
-      make_bias_map(&mb, p, dtype))
-    bias_mode = 2;
+  if (bias_mode == 2 && !make_bias_map(&mb, p, dtype)) bias_mode = 1;
   if ((bias_mode == 0 || bias_mode == 2) && short_preferred(p)) return launch_short(p, dtype, mq, mb, num_sms, stream);
   CUtensorMap mo;
   if (!make_out_map(&mo, p, dtype)) return cudaErrorNotSupported;

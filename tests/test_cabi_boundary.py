@@ -69,9 +69,11 @@ def test_workspace_size_and_kernel_choice():
     assert need >= 256 + 8 * 4 * (1000 // 256 + 8) and need % 256 == 0
     assert cabi.kernel_kind(_args(dtype=torch.float32)) == 0
     assert cabi.workspace_size(_args(dtype=torch.float32)) == 256
-    assert cabi.kernel_kind(_args(D=96, Dv=96)) == 0    # head dim without a tensor-core instance
+    assert cabi.kernel_kind(_args(D=96, Dv=96)) == 1    # narrower than the tile
     assert cabi.kernel_kind(_args(D=64, Dv=64)) == 1
-    assert cabi.kernel_kind(_args(D=128, Dv=64)) == 0   # dim_qk != dim_v
+    assert cabi.kernel_kind(_args(D=128, Dv=64)) == 1   # dim_qk != dim_v
+    assert cabi.kernel_kind(_args(D=256, Dv=256)) == 0  # accumulators beyond the tensor memory
+    assert cabi.kernel_kind(_args(D=100, Dv=64)) == 0   # rows TMA cannot address
     assert cabi.kernel_kind(_args(flags=cabi.FLAG_FORCE_GENERIC)) == 0
     assert cabi.kernel_kind(_args(dtype=torch.float16, H=8, Hk=2)) == 1
 

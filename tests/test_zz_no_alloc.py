@@ -62,6 +62,20 @@ def test_static_scratch_entry_point_rejects_oversized_work_lists():
     torch.cuda.synchronize()
 
 
+def test_static_scratch_entry_point_runs_narrow_head_dims_without_a_list():
+    """Head dims that are not 64 or 128 go to the CUDA-core kernel, which needs no list, where the list does not fit; the
+    regular entry point gives the tensor-core kernel's result for the same call."""
+    B = 70000
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    q, k, v = (torch.randn(B, 16, d, generator=gen, device="cuda").to(torch.bfloat16) for d in (32, 32, 16))
+    off = torch.arange(B + 1, dtype=torch.int64, device="cuda")
+    out = torch.full_like(v, float("nan"))
+    cabi.hstu_jagged_forward_static(q, k, v, out, None, None, 0, 16, 1.0, off, None, None, 0, 0.25)
+    want = cabi.hstu_jagged_forward(q, k, v, None, None, 0, 16, 1.0, off, None, None, 0, 0.25)
+    # P is rounded to bf16 after 32-bit sums in another order, and the output once more: two units in the last place
+    torch.testing.assert_close(out.float(), want.float(), rtol=2.0**-6, atol=1e-5)
+
+
 def test_static_scratch_entry_point_reports_the_device_status_word():
     # inconsistent offsets are flagged in the status word of the built-in block (and nothing faults)
     args = _cuda(make_case(4, 2, 2, 64, 64, 10, 200, torch.bfloat16, seed=43))
