@@ -575,18 +575,35 @@ cudaError_t launch_inst(const KParams& p, const CUtensorMap& mq, const CUtensorM
 //            hstu_paged, 16-80 queries per sequence: 512 of mean 1000: 238 -> 184; 64 of 1000: 53 -> 61
 //   D = 128  8700 of mean 60: 649 -> 481; 3500 of mean 150: 460 -> 487; 220 of 2400: 1453 -> 2105
 //            hstu_paged: 2048 of mean 300: 510 -> 433; 512 of 1000: 292 -> 270; 8 of 1000: 38 -> 44
-static bool short_rule(const KParams& p, long long mean_k) {
+//
+// Means do not show a single long sequence, whose chain is what such a batch then waits for: its last Q tile - both of a
+// pair, one after the other, in calls of many items - takes 1.65 us per 64 keys here, 125 us of 8192 keys there.  So the
+// longest chain the call allows has to fit the time the other kernel needs for the batch as such, about 2 us a pair and
+// 9 us per 1000 keys of its sequences on each SM; with hstu_paged that kernel has the gather in front of it.  (max_seq_len_k
+// stands for the longest length, which only the device knows.)  D = 64, 512 sequences of mean 80: 36 here, 47 there; and one
+// more of 1024: 39 / 49, of 2048: 65 / 53, of 8192: 234 / 157; 2048 of mean 80 and one of 2048: 122 / 157, of 4096:
+// 206 / 172; 1024 of mean 300 and one of 2048: 193 / 249, of 8192: 409 / 313; 300 of mean 800 and one of 8192: 271 / 330.
+// hstu_paged, 512 of mean 350 and one of 4096: 104 / 126, of 16384: 306 / 224.  Up to 160 keys the two differ by 0.5 us
+// whatever the batch.
+static bool short_rule(const KParams& p, long long mean_k, bool in_place) {
   const bool wide = p.dqk > 64 || p.dv > 64;
   const long long mean_q = p.total_q / p.batch;
-  if (mean_k < (wide ? 96 : 320)) return true;
-  const long long tiles = p.hq * (p.total_q / kTileM > p.batch ? p.total_q / kTileM : p.batch);
-  if (tiles < kFewItems) return false;
-  return mean_q < 96 || (!wide && mean_k < 1024);
+  if (mean_k >= (wide ? 96 : 320)) {
+    const long long tiles = p.hq * (p.total_q / kTileM > p.batch ? p.total_q / kTileM : p.batch);
+    if (tiles < kFewItems) return false;
+    if (mean_q >= 96 && (wide || mean_k >= 1024)) return false;
+  }
+  if (p.maxk <= 160) return true;
+  const long long in_pairs = p.total_q / kPairM + p.batch / 2;
+  const double pairs = static_cast<double>(p.hq) * (in_pairs > p.batch ? in_pairs : p.batch);
+  const bool many = pairs >= 8.0 * 148 * (wide ? 2 : p.bias ? 3 : 4) && p.maxq > kTileM;
+  const double chain_us = p.maxk * (in_place ? 0.011 : many ? 0.05 : 0.026);
+  return chain_us <= (in_place ? 4.0 : 0.0) + pairs / 148 * (2.0 + 0.009 * mean_k);
 }
 bool short_preferred(const KParams& p) {
   if (p.paged_split) return true;                     // (decided by short_paged_split)
   if (p.batch <= 0 || p.paged_direct) return false;   // (cache pages beside staging tensors: hstu_tc.cu)
-  return short_rule(p, p.total_k / p.batch);
+  return short_rule(p, p.total_k / p.batch, false);
 }
 
 // Whether an hstu_paged call can run here without staging anything: K / V tiles of 64 keys lie in one page, and no bias - a
@@ -598,7 +615,7 @@ bool short_paged_split(const KParams& p) {
       p.num_pages > 0x7fffff00ll / 2 / p.page_size)
     return false;
   // (the cached keys are not known here: all pages, each sequence's last one half full)
-  return short_rule(p, (p.num_page_ids * p.page_size + p.total_q) / p.batch - p.page_size / 2);
+  return short_rule(p, (p.num_page_ids * p.page_size + p.total_q) / p.batch - p.page_size / 2, true);
 }
 
 // Returns cudaSuccess, a CUDA error, or cudaErrorNotSupported when a tensor map could not be encoded.

@@ -78,6 +78,21 @@ def test_workspace_size_and_kernel_choice():
     assert cabi.kernel_kind(_args(dtype=torch.float16, H=8, Hk=2)) == 1
 
 
+@pytest.mark.parametrize("batch,mean,max_seq_len,D,short", [
+    # many short sequences: the longest one the call allows fits the time of the batch, or does not
+    (512, 80, 160, 64, 1), (512, 80, 1024, 64, 1), (512, 80, 2048, 64, 0), (2048, 80, 2048, 64, 1), (2048, 80, 4096, 64, 0),
+    (1024, 300, 2048, 64, 1), (1024, 300, 8192, 64, 0), (300, 800, 8192, 64, 1), (512, 60, 1024, 128, 1), (2048, 60, 4096, 128, 0),
+    # few
+    (8, 80, 160, 64, 1), (32, 300, 400, 64, 0), (8, 80, 8192, 64, 0), (10, 800, 1100, 64, 0),
+    # not short
+    (1024, 300, 400, 128, 0), (300, 2000, 4096, 64, 0)])
+def test_short_form_and_the_longest_sequence(batch, mean, max_seq_len, D, short):
+    """Which forward kernel a batch goes to, on the two sides of the rule's lines (csrc/hstu_short.cu gives the times)."""
+    q = _Fake(batch * mean, 4, D)
+    a, _ = cabi.make_args(q, q, q, None, _Fake(batch + 1, dtype=torch.int64), max_seq_len=max_seq_len, ptr=lambda t: t._addr)
+    assert cabi.kernel_kind(a) == 1 and cabi.short_form(a) == short
+
+
 @pytest.mark.parametrize("kw,needle", [
     (dict(mask_type=1), "triu"),
     (dict(mask_type=4), "maskType expect in [0, 3]"),

@@ -5,7 +5,7 @@ import torch
 
 from oracle import hstu_paged_oracle as PO
 from ops_rec_b200 import cabi
-from tests._parity import assert_parity, run_cabi
+from tests._parity import assert_parity, run_cabi, to_cuda
 from tests._util import make_case
 from tests.test_paged import make_paged_case
 
@@ -14,12 +14,23 @@ pytestmark = pytest.mark.gpu
 BF16, FP16 = torch.bfloat16, torch.float16
 
 
+def run(args, short=True):
+    """The call's output; it has to run on the kernel for short sequences (`short`), or on the other one."""
+    cu = to_cuda(args)
+    a, keep = cabi.make_args(cu["q"], cu["k"], cu["v"], None, cu["seq_offset"],
+                             **{n: cu[n] for n in ("mask", "attn_bias", "mask_type", "max_seq_len", "max_seq_len_k",
+                                                   "seq_offset_k", "num_context", "num_target", "target_group_size", "alpha")})
+    assert cabi.kernel_kind(a) == 1 and cabi.short_form(a) == short
+    return run_cabi(args)
+
+
 @pytest.mark.parametrize("dims", [(64, 64), (8, 16), (48, 32)])
 @pytest.mark.parametrize("L", [1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 191, 192, 193, 257, 319])
 @pytest.mark.parametrize("dtype,rab", [(BF16, None), (FP16, "batch"), (BF16, "shared3")])
 def test_lengths(dims, L, dtype, rab):
-    args = make_case(3, 4, 2, *dims, L, L, dtype, seed=L, rab=rab, max_seq_len=(L + 7) // 8 * 8)
-    out, status = run_cabi(args)
+    batch = 3 if L <= 160 else 48   # (a few longer sequences go to the other kernel)
+    args = make_case(batch, 4, 2, *dims, L, L, dtype, seed=L, rab=rab, max_seq_len=(L + 7) // 8 * 8)
+    out, status = run(args)
     assert status == 0
     assert_parity(out, args, label=f"{dims} {L}")
 
@@ -29,7 +40,7 @@ def test_lengths(dims, L, dtype, rab):
                                       (20, 60, dict(tgt=9, g=2, ctx=3, rab="batch", delta=True))])
 def test_wide(dims, lo, hi, kw):
     args = make_case(7, 4, 2, *dims, lo, hi, BF16, seed=hi, max_seq_len=96, **kw)
-    out, status = run_cabi(args)
+    out, status = run(args)
     assert status == 0
     assert_parity(out, args, label=f"{dims} {hi}")
 
@@ -38,16 +49,18 @@ def test_wide(dims, lo, hi, kw):
 def test_many_items(rab, tgt):
     """More work items than eight per CTA: pairs of Q tiles, look-ups spread over the tiles before."""
     args = make_case(2600, 2, 2, 32, 32, 1, 150, BF16, seed=1, rab=rab, tgt=tgt, g=1 if tgt else 0, max_seq_len=160)
-    out, status = run_cabi(args)
+    out, status = run(args)
     assert status == 0
     assert_parity(out, args)
 
 
-@pytest.mark.parametrize("batch,lo,hi", [(40, 300, 339), (300, 500, 1100), (10, 500, 1100)])
-def test_around_the_rule(batch, lo, hi):
+@pytest.mark.parametrize("batch,lo,hi,max_seq_len,short", [
+    (24, 300, 339, None, False), (60, 280, 315, None, True), (300, 500, 1100, None, True), (10, 500, 1100, None, False),
+    (20, 40, 80, 160, True), (20, 40, 80, 168, False), (80, 40, 80, 168, True), (80, 40, 80, 1024, False)])
+def test_around_the_rule(batch, lo, hi, max_seq_len, short):
     """Both sides of the rule's lines give the oracle's result."""
-    args = make_case(batch, 4, 4, 64, 64, lo, hi, BF16, seed=batch)
-    out, status = run_cabi(args)
+    args = make_case(batch, 4, 4, 64, 64, lo, hi, BF16, seed=batch, max_seq_len=max_seq_len)
+    out, status = run(args, short)
     assert status == 0
     assert_parity(out, args)
 
@@ -57,14 +70,14 @@ def test_around_the_rule(batch, lo, hi):
 def test_neighbours_never_leak(poison, D):
     """Rows of the other sequences may hold anything."""
     args = make_case(5, 2, 2, D, D, 70, 90, BF16, seed=2)
-    want, _ = run_cabi(args)
+    want, _ = run(args)
     off = args["seq_offset"].tolist()
     for n in ("q", "k", "v"):
         t = args[n].clone()
         t[:off[2]] = poison
         t[off[3]:] = poison
         args[n] = t
-    out, status = run_cabi(args)
+    out, status = run(args)
     assert status == 0
     assert torch.equal(out[off[2]:off[3]], want[off[2]:off[3]])
 
