@@ -22,6 +22,9 @@ HSTU_API int hstu_debug_tiles_host(int32_t len_q, int32_t len_k, int32_t num_con
                           int32_t target_group_size, int32_t mask_type, int32_t r0, int32_t rows, int32_t bn,
                           uint64_t* full_bits);
 
+/* out[i] = a[i] / b[i], fp32 device arrays, by the quotient of the fp32 kernels' SiLU and sigmoid (b >= 1). */
+HSTU_API int hstu_debug_divide(const void* a, const void* b, void* out, int64_t n, void* stream);
+
 /* Whether phase 2 of the forward would run the kernel for batches of short sequences (1) or another one (0) for these
  * arguments; negative = error code. */
 HSTU_API int hstu_debug_short_form(const HstuJaggedArgs* args);

@@ -23,7 +23,7 @@ ST_BAD_OFFSETS, ST_LEN_GT_MAX, ST_BAD_CTX_TARGET, ST_BAD_PAGES, ST_PIPE_TIMEOUT 
 EXPORTS = (
     "hstu_jagged_fwd_get_workspace_size", "hstu_jagged_fwd", "hstu_jagged_fwd_status",
     "hstu_jagged_fwd_kernel_kind", "hstu_plan_host", "hstu_debug_mask_host", "hstu_debug_tiles_host",
-    "hstu_debug_short_form",
+    "hstu_debug_short_form", "hstu_debug_divide",
     "hstu_last_error", "hstu_b200_version", "hstu_jagged_fwd_static", "hstu_jagged_fwd_static_status",
     "hstu_jagged_bwd_get_workspace_size", "hstu_jagged_bwd", "ops_rec_ln_mul_f32", "ops_rec_in_linear_silu_fwd",
     "hstu_paged_fwd_get_workspace_size", "hstu_paged_fwd",
@@ -116,6 +116,8 @@ def load():
     lib.hstu_plan_host.argtypes = [A, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
                                    C.POINTER(C.c_uint32)]
     lib.hstu_plan_host.restype = C.c_int64
+    lib.hstu_debug_divide.argtypes = [C.c_void_p] * 3 + [C.c_int64, C.c_void_p]
+    lib.hstu_debug_divide.restype = C.c_int
     lib.hstu_debug_short_form.argtypes = [A]
     lib.hstu_debug_short_form.restype = C.c_int
     lib.hstu_debug_mask_host.argtypes = [C.c_int32] * 6 + [C.c_void_p]
@@ -220,6 +222,12 @@ def workspace_size(args):
 
 def kernel_kind(args):
     return check(load().hstu_jagged_fwd_kernel_kind(C.byref(args)))
+
+
+def debug_divide(a, b):
+    out = a.new_empty(a.shape)
+    check(load().hstu_debug_divide(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel(), None))
+    return out
 
 
 def short_form(args):

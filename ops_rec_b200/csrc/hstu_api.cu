@@ -21,6 +21,7 @@ bool tc_supported(const KParams& p, int dtype);
 bool short_paged_split(const KParams& p);
 bool tc_runs_short(const KParams& p);
 cudaError_t launch_tc(const KParams& p, int dtype, int num_sms, cudaStream_t stream);
+cudaError_t launch_divide(const float* a, const float* b, float* out, long long n, cudaStream_t stream);
 cudaError_t launch_bwd_generic(const BwdParams& bp, int dtype, cudaStream_t stream);
 bool bwd_tc_supported(const BwdParams& bp, int dtype);
 cudaError_t launch_bwd_tc(const BwdParams& bp, int dtype, int num_sms, cudaStream_t stream);
@@ -655,6 +656,14 @@ int hstu_debug_mask_host(int32_t len_q, int32_t len_k, int32_t num_context, int3
 
 // For the q-tile of rows [r0, r0 + rows): number of K tiles of width bn to visit, and (bit t of full_bits,
 // t < 64) whether K tile t is classified "no predicate needed".
+int hstu_debug_divide(const void* a, const void* b, void* out, int64_t n, void* stream) {
+  g_err[0] = 0;
+  if (!a || !b || !out) return fail(HSTU_E_NULL, "a / b / out is null");
+  const cudaError_t e = hstu::launch_divide(static_cast<const float*>(a), static_cast<const float*>(b), static_cast<float*>(out),
+                                            n, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? HSTU_OK : fail(HSTU_E_CUDA, "kernel launch: %s", cudaGetErrorString(e));
+}
+
 int hstu_debug_short_form(const HstuJaggedArgs* args) {
   const int kind = hstu_jagged_fwd_kernel_kind(args);
   return kind == 1 ? (hstu::tc_runs_short(to_params(args, nullptr, 0)) ? 1 : 0) : kind;

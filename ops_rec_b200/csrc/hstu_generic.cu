@@ -282,6 +282,10 @@ bool simt_supported(const KParams& p, int dtype) {
          simt::aligned_to(p.v, dtype) && simt::aligned_to(p.out, dtype);
 }
 
+__global__ void divide_kernel(const float* a, const float* b, float* out, long long n) {
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += gridDim.x * 256ll) out[i] = simt::divide(a[i], b[i]);
+}
+
 template <typename T>
 cudaError_t launch_t(const KParams& p, int dtype, cudaStream_t stream) {
   if (simt_supported(p, dtype)) {
@@ -301,6 +305,12 @@ cudaError_t launch_t(const KParams& p, int dtype, cudaStream_t stream) {
 }
 
 }  // namespace
+
+// simt::divide on arrays, for the tests
+cudaError_t launch_divide(const float* a, const float* b, float* out, long long n, cudaStream_t stream) {
+  divide_kernel<<<256, 256, 0, stream>>>(a, b, out, n);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_generic(const KParams& p, int dtype, cudaStream_t stream) {
   switch (dtype) {

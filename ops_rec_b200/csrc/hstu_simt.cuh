@@ -33,8 +33,13 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(f
 template <> __device__ __forceinline__ __half from_float<__half>(float x) { return __float2half_rn(x); }
 template <typename T> __device__ __forceinline__ float rounded(float x) { return to_float<T>(from_float<T>(x)); }
 
-// a / b (b >= 1) without the slow path of an IEEE division: the reciprocal, and one correction of the quotient from its
-// remainder, which leaves it within an ulp.  (An infinite b or a keeps the uncorrected quotient.)
+// a / b for b >= 1 with the remainder correction of Markstein ("Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  r = (1 + d) / b with |d| <= 2^-23 (the documented error of rcp.approx), so q = a r is
+// within 2^-22 of a / b; its remainder a - q b comes exact out of one FMA, and q + rem r = a / b up to |d| 2^-22 |a / b|
+// before the one rounding at the end: half an ulp, and 2^-21 of one.  (Beyond b = 2^126 r is subnormal, which costs up to
+// two bits of d: half an ulp, and 2^-17 of one.)  An infinite a or b keeps the uncorrected quotient: what the division
+// gives; a zero comes out positive.  The division itself costs 16 % of a training step in fp32 (157 -> 182 us) and changes no error: against 64 bits
+// it is the sums of a row that count.
 __device__ __forceinline__ float divide(float a, float b) {
   float r;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b));

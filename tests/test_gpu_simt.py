@@ -3,6 +3,7 @@ the edges of their 32-row / 64-key tiles and of their head dims; tolerances as i
 import pytest
 import torch
 
+from ops_rec_b200 import cabi
 from tests._parity import assert_parity, run_cabi
 from tests._util import make_case
 from tests.test_gpu_backward import assert_bwd_parity, make_bwd_case, run_bwd
@@ -45,3 +46,27 @@ def test_misaligned_rows_take_the_other_kernel():
     out, status = run_cabi(moved)
     assert status == 0
     torch.testing.assert_close(out, want, rtol=1e-5, atol=1e-6)
+
+
+def test_quotient():
+    """The quotient of the SiLU and the sigmoid is within half an ulp and 2^-17 of one of a / b for every b >= 1 (the bound
+    beside the function), and the division's for infinities and NaN."""
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    n = 1 << 22
+    a = torch.randn(n, generator=gen, device="cuda") * torch.exp2(torch.rand(n, generator=gen, device="cuda") * 40 - 20)
+    b = torch.exp2(torch.rand(n, generator=gen, device="cuda") * 127.99).clamp_(min=1)
+    b[: n // 4] = 1 + torch.rand(n // 4, generator=gen, device="cuda")          # sigmoids of positive scores
+    a[n // 8: n // 4] = 1
+    a[n // 2: 3 * n // 4] = -torch.log(b[n // 2: 3 * n // 4] - 1).clamp_(min=-80, max=89)   # SiLU: x / (1 + exp(-x))
+    got, want = cabi.debug_divide(a, b).double(), a.double() / b.double()
+    ulp = torch.exp2(torch.floor(torch.log2(want.abs().clamp(min=2.0**-126))) - 23)
+    normal = want.abs() >= 2.0**-126
+    assert ((got - want).abs()[normal] <= (0.5 + 2.0**-17) * ulp[normal]).all()
+    assert ((got - want).abs()[~normal] <= 2.0**-149).all()
+    assert (got.float() != want.float()).float().mean() < 1e-5
+    inf, nan = float("inf"), float("nan")
+    x, y = (t.flatten().contiguous().cuda() for t in torch.meshgrid(
+        torch.tensor([0.0, -0.0, 1.0, -88.0, inf, -inf, nan]), torch.tensor([1.0, 3.0, 2.0**127, inf, nan]), indexing="ij"))
+    got, want = cabi.debug_divide(x, y), x / y
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.nan_to_num(9), want.nan_to_num(9))
