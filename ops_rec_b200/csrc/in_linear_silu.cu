@@ -47,6 +47,7 @@ constexpr long long kLsWaitLimit = 2000000000ll;
 struct LsBars {
   uint64_t full[kLsStages], empty[kLsStages];
   uint64_t acc_full[2], acc_free[2];   // per accumulator buffer (acc_free: the leader's counts both CTAs' epilogue warps)
+  uint64_t done;   // every product this pair has issued is complete
   uint32_t tmem_base;
   int abort_flag;
   int epi_stop[2];   // the abort flag as the epilogue warps agree to have seen it (per tile parity)
@@ -154,6 +155,7 @@ in_linear_silu_kernel(const LinSiluParams p, const __grid_constant__ CUtensorMap
       ptx::mbar_init(ptx::smem_u32(&bars->acc_full[i]), 1);
       ptx::mbar_init(ptx::smem_u32(&bars->acc_free[i]), 2 * 8);   // every epilogue warp of the pair
     }
+    ptx::mbar_init(ptx::smem_u32(&bars->done), 1);
     bars->abort_flag = 0;
     ptx::fence_mbar_init();
   }
@@ -199,8 +201,13 @@ in_linear_silu_kernel(const LinSiluParams p, const __grid_constant__ CUtensorMap
         }
         if (*reinterpret_cast<volatile int*>(&bars->abort_flag)) break;
       }
-      // drain (matters only after an abort): the last loads - the leader's barriers count those of both CTAs - have
-      // landed before either CTA leaves the cluster barrier at the end
+      // drain (matters only after an abort): the last loads have landed before either CTA leaves the cluster barrier at the
+      // end.  The leader's barriers count those of both CTAs, but the other CTA may have requested more than the leader
+      // has, on barriers it cannot wait for: it gives them a millisecond.
+      if (rank != 0 && *reinterpret_cast<volatile int*>(&bars->abort_flag)) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000ll) {}
+      }
       if (rank == 0) {
         for (uint32_t back = 0; back < kLsStages && back < g; ++back) {
           const uint32_t c = g - 1 - back;
@@ -242,6 +249,7 @@ in_linear_silu_kernel(const LinSiluParams p, const __grid_constant__ CUtensorMap
         if (*reinterpret_cast<volatile int*>(&bars->abort_flag)) break;
         ptx::mma_commit_pair(ptx::smem_u32(&bars->acc_full[buf]));
       }
+      ptx::mma_commit_pair(ptx::smem_u32(&bars->done));
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ epilogue (thread = row of the tile)
@@ -358,6 +366,10 @@ in_linear_silu_kernel(const LinSiluParams p, const __grid_constant__ CUtensorMap
 
   ptx::tc_fence_before();
   __syncthreads();
+  // (matters only after an abort: otherwise the epilogues have waited for every product)
+  if (tid == 0)
+    for (int spin = 0; spin < (1 << 22) && !ptx::mbar_try_wait(ptx::smem_u32(&bars->done), 0); ++spin) {}
+  __syncwarp();
   ptx::cluster_sync();   // neither CTA leaves while the other's loads, products or arrivals may still touch it
   if (warp == 2) {
     ptx::tc_fence_after();
