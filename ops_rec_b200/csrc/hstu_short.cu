@@ -583,8 +583,8 @@ cudaError_t launch_inst(const KParams& p, const CUtensorMap& mq, const CUtensorM
 // stands for the longest length, which only the device knows.)  D = 64, 512 sequences of mean 80: 36 here, 47 there; and one
 // more of 1024: 39 / 49, of 2048: 65 / 53, of 8192: 234 / 157; 2048 of mean 80 and one of 2048: 122 / 157, of 4096:
 // 206 / 172; 1024 of mean 300 and one of 2048: 193 / 249, of 8192: 409 / 313; 300 of mean 800 and one of 8192: 271 / 330.
-// hstu_paged, 512 of mean 350 and one of 4096: 104 / 126, of 16384: 306 / 224.  Up to 160 keys the two differ by 0.5 us
-// whatever the batch.
+// hstu_paged, 512 of mean 350 and one of 4096: 104 / 126, of 16384: 306 / 224.  No call takes the other kernel less than
+// some 5.5 us beside its launches: a few sequences of at most 192 rows 10.6 here, 11.5 there; of 256: 12.3 / 11.7.
 static bool short_rule(const KParams& p, long long mean_k, bool in_place) {
   const bool wide = p.dqk > 64 || p.dv > 64;
   const long long mean_q = p.total_q / p.batch;
@@ -593,12 +593,12 @@ static bool short_rule(const KParams& p, long long mean_k, bool in_place) {
     if (tiles < kFewItems) return false;
     if (mean_q >= 96 && (wide || mean_k >= 1024)) return false;
   }
-  if (p.maxk <= 160) return true;
   const long long in_pairs = p.total_q / kPairM + p.batch / 2;
   const double pairs = static_cast<double>(p.hq) * (in_pairs > p.batch ? in_pairs : p.batch);
   const bool many = pairs >= 8.0 * 148 * (wide ? 2 : p.bias ? 3 : 4) && p.maxq > kTileM;
   const double chain_us = p.maxk * (in_place ? 0.011 : many ? 0.05 : 0.026);
-  return chain_us <= (in_place ? 4.0 : 0.0) + pairs / 148 * (2.0 + 0.009 * mean_k);
+  const double batch_us = (in_place ? 4.0 : 0.0) + pairs / 148 * (2.0 + 0.009 * mean_k);
+  return chain_us <= (batch_us > 5.5 ? batch_us : 5.5);
 }
 bool short_preferred(const KParams& p) {
   if (p.paged_split) return true;                     // (decided by short_paged_split)

@@ -83,7 +83,7 @@ def test_workspace_size_and_kernel_choice():
     (512, 80, 160, 64, 1), (512, 80, 1024, 64, 1), (512, 80, 2048, 64, 0), (2048, 80, 2048, 64, 1), (2048, 80, 4096, 64, 0),
     (1024, 300, 2048, 64, 1), (1024, 300, 8192, 64, 0), (300, 800, 8192, 64, 1), (512, 60, 1024, 128, 1), (2048, 60, 4096, 128, 0),
     # few
-    (8, 80, 160, 64, 1), (32, 300, 400, 64, 0), (8, 80, 8192, 64, 0), (10, 800, 1100, 64, 0),
+    (8, 80, 208, 64, 1), (8, 80, 216, 64, 0), (32, 300, 400, 64, 0), (8, 80, 8192, 64, 0), (10, 800, 1100, 64, 0),
     # not short
     (1024, 300, 400, 128, 0), (300, 2000, 4096, 64, 0)])
 def test_short_form_and_the_longest_sequence(batch, mean, max_seq_len, D, short):

@@ -56,7 +56,7 @@ def test_many_items(rab, tgt):
 
 @pytest.mark.parametrize("batch,lo,hi,max_seq_len,short", [
     (24, 300, 339, None, False), (60, 280, 315, None, True), (300, 500, 1100, None, True), (10, 500, 1100, None, False),
-    (20, 40, 80, 160, True), (20, 40, 80, 168, False), (80, 40, 80, 168, True), (80, 40, 80, 1024, False)])
+    (20, 40, 80, 208, True), (20, 40, 80, 216, False), (120, 40, 80, 216, True), (120, 40, 80, 1024, False)])
 def test_around_the_rule(batch, lo, hi, max_seq_len, short):
     """Both sides of the rule's lines give the oracle's result."""
     args = make_case(batch, 4, 4, 64, 64, lo, hi, BF16, seed=batch, max_seq_len=max_seq_len)
