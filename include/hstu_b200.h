@@ -168,7 +168,9 @@ HSTU_API int hstu_jagged_fwd_static_status(void* stream, uint32_t* status);
  *   seq_offset_t    [batch + 1] offsets of num_target; implied by num_target and not read (may be null)
  * Workspace (phase 1 sizes it): the forward's work list plus two staging tensors of
  * (num_page_ids * page_size + total_q + 128) rows into which one gather pass packs the keys and values; the
- * attention itself is then the jagged forward in its delta form on the same kernels.  batch <= 65535. */
+ * attention itself is then the jagged forward in its delta form on the same kernels.  (Calls whose pages and new rows are
+ * read where they lie - short sequences, page sizes that are multiples of 64, no bias - leave the staging tensors unused;
+ * the size is the same, it does not depend on the pointers.)  batch <= 65535. */
 typedef struct HstuPagedArgs {
   uint32_t struct_bytes;  /* sizeof(HstuPagedArgs) */
   int32_t page_size;

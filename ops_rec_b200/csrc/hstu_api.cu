@@ -342,7 +342,7 @@ int hstu_paged_fwd(const HstuPagedArgs* args, void* workspace, uint64_t workspac
   p.k_new = b->k;
   p.v_new = b->v;
   // Batches of short sequences or few queries: the kernel reads cache pages and new rows where they lie.  (4096 users of
-  // mean 271 cached rows: the gather of partial pages and new rows took 192 of 540 us.)  Otherwise whole 128-row pages go
+  // mean 271 cached rows: 386 us, 540 with a gather of partial pages and new rows in front of it.)  Otherwise whole 128-row pages go
   // from the cache straight into the tensor-core kernel's K / V ring and the rest through the staging tensors.
   const bool tc = wants_tc(&pl.fwd, p);
   p.paged_split = tc && hstu::short_paged_split(p) ? 1 : 0;

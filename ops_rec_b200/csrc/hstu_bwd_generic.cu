@@ -48,13 +48,13 @@ __device__ __forceinline__ void load_tile(float* dst, int ld, const T* src, long
   }
 }
 
-// P (rounded) and dS (rounded) of element (i, j) from the raw dot products s = q_i.k_j and dp = dO_i.v_j.
-// d_bias gets dS for the reference's x = alpha (S + bias) and dX for the alpha-before-bias variant.
 template <typename T>
 __device__ __forceinline__ float bias_at(const KParams& p, int b, int h, int i, int j) {
   return ld_f<T>(static_cast<const T*>(p.bias) + static_cast<long long>(b) * p.bias_bstride +
                  (static_cast<long long>(h) * p.maxq + i) * p.maxk + j);
 }
+// P (rounded) and dS (rounded) of element (i, j) from the raw dot products s = q_i.k_j and dp = dO_i.v_j.
+// d_bias gets dS for the reference's x = alpha (S + bias) and dX for the alpha-before-bias variant.
 // bv: bias_at(i, j) of a visible element (unused without a bias)
 template <typename T>
 __device__ __forceinline__ void score_grad(const KParams& p, int b, int h, int i, int j, bool visible, float s, float dp,

@@ -53,9 +53,6 @@ template <> struct BPack<__nv_bfloat16> {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
   }
-  static __device__ __forceinline__ float one(const void* p, long long i) {
-    return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
-  }
   static __device__ __forceinline__ float2 unpack(uint32_t u) {
     return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
   }
@@ -70,9 +67,6 @@ template <> struct BPack<__half> {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
   }
-  static __device__ __forceinline__ float one(const void* p, long long i) {
-    return __half2float(static_cast<const __half*>(p)[i]);
-  }
   static __device__ __forceinline__ float2 unpack(uint32_t u) {
     return __half22float2(*reinterpret_cast<__half2*>(&u));
   }
@@ -81,7 +75,7 @@ template <> struct BPack<__half> {
 struct BwdBars {
   uint64_t a_full;             // the resident pair has landed
   uint64_t b1_full[3], b1_free[3];   // the streamed tiles, a ring each
-  uint64_t b2_full[3], b2_free[3];
+  uint64_t b2_full[2], b2_free[2];
   uint64_t t1_full[2];         // T1 (the scores) of an even / odd step is complete
   uint64_t t2_full;            // T2 (dP) of the current step is complete
   uint64_t p_full[2];          // dK/dV pass: P is written, first / second 32 values of each 64 (256 arrivals)
@@ -178,8 +172,7 @@ __device__ __forceinline__ float2 score_part(float2 s, float2 bias, float alpha,
   return f;
 }
 
-// kStaged (dK/dV pass with a bias that TMA can tile): a kernel of its own - the same code merely present in the
-// bias-free kernel cost that one 4 %.
+// Slots of the two rings of streamed tiles (the kernel says why), and the shared memory of a CTA.
 template <int D, bool kStaged, bool kDKV> struct BwdRings {
   static constexpr int k1 = kDKV || (D == 128 && kStaged) ? 2 : 3, k2 = 2;
   static constexpr int kSmem = 1024 + (2 + k1 + k2) * (D / 64) * kTileM * 128 + (kStaged ? 2 * kTileM * 128 : 0) + 512;
@@ -187,6 +180,8 @@ template <int D, bool kStaged, bool kDKV> struct BwdRings {
 };
 static_assert(sizeof(BwdBars) <= 512, "barrier block too large");
 
+// kStaged (a bias that TMA can tile): a kernel of its own - the same code merely present in the bias-free kernel cost that
+// one 4 %.
 template <int D, typename T, bool kDKV, bool kStaged>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1,
@@ -241,11 +236,11 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
     for (int i = 0; i < 3; ++i) {
       ptx::mbar_init(ptx::smem_u32(&bars->b1_full[i]), 1);
       ptx::mbar_init(ptx::smem_u32(&bars->b1_free[i]), 1);
-      ptx::mbar_init(ptx::smem_u32(&bars->b2_full[i]), 1);
-      ptx::mbar_init(ptx::smem_u32(&bars->b2_free[i]), 1);
     }
     ptx::mbar_init(ptx::smem_u32(&bars->t2_full), 1);
     for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(ptx::smem_u32(&bars->b2_full[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&bars->b2_free[i]), 1);
       ptx::mbar_init(ptx::smem_u32(&bars->t1_full[i]), 1);
       ptx::mbar_init(ptx::smem_u32(&bars->p_full[i]), 2 * kTileM);
       ptx::mbar_init(ptx::smem_u32(&bars->u_full[i]), 2 * kTileM);
@@ -285,8 +280,8 @@ hstu_bwd_tc_kernel(const BwdParams bp, const __grid_constant__ CUtensorMap tm_a1
   // requested the last loads of a tile it draws the next one, publishes it in one of two slots (item_full / item_free)
   // and - once the MMAs of the current tile are complete (acc_full: the resident pair's buffer is free) - requests
   // the next tile's loads, so that the draw (an atomic and a dependent load of the list entry) and the first loads
-  // overlap the current tile's epilogue.  The draw comes a step or two before the current tile's end (the ring of
-  // streamed tiles has two stages), which costs no balance worth the name; drawing at the START of the current tile
+  // overlap the current tile's epilogue.  The draw comes two or three steps before the current tile's end (as many as the
+  // rings of streamed tiles have slots), which costs no balance worth the name; drawing at the START of the current tile
   // did (a tile drawn early is a tile that cannot go to a CTA that has run dry: - 7 % on a batch with four tiles per
   // CTA).
   // The other warps meet at a named barrier at the end of a tile (the producer warp takes no part in it).
@@ -857,7 +852,6 @@ cudaError_t launch_bwd_tc_t(const BwdParams& bp, int dtype, int num_sms, cudaStr
   const int bias_staged = p.bias && (p.maxk % 8 == 0) && (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0 &&
                           p.bias_bstride == static_cast<long long>(p.hq) * p.maxq * p.maxk &&
                           make_bias_tile_map(&mb, p, dtype);
-  // one pass: the instantiation for (staged bias, tile look-ahead), its shared-memory size set, launched
   bool overlap = false;
   // one pass: the instantiation with or without a staged bias, its shared-memory size set, launched
   auto launch = [&](auto kdkv, long long tiles_bound, const CUtensorMap& a1, const CUtensorMap& a2,

@@ -57,9 +57,6 @@ template <> struct Pack<__nv_bfloat16> {
   static __device__ __forceinline__ float2 unpack(uint32_t u) {
     return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
   }
-  static __device__ __forceinline__ float one(const void* p, long long i) {
-    return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
-  }
 };
 template <> struct Pack<Bf16Exp> : Pack<__nv_bfloat16> {
   static constexpr bool kExact = true;    // SiLU: exp2 and reciprocal
@@ -73,9 +70,6 @@ template <> struct Pack<__half> {
   }
   static __device__ __forceinline__ float2 unpack(uint32_t u) {
     return __half22float2(*reinterpret_cast<__half2*>(&u));
-  }
-  static __device__ __forceinline__ float one(const void* p, long long i) {
-    return __half2float(static_cast<const __half*>(p)[i]);
   }
 };
 

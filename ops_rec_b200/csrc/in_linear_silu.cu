@@ -56,7 +56,6 @@ struct LsBars {
 template <typename T> struct LsPack;
 template <> struct LsPack<__nv_bfloat16> {
   static constexpr int kFormat = 1;
-  static __device__ __forceinline__ float round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -74,7 +73,6 @@ template <> struct LsPack<__nv_bfloat16> {
 };
 template <> struct LsPack<__half> {
   static constexpr int kFormat = 0;
-  static __device__ __forceinline__ float round(float x) { return __half2float(__float2half_rn(x)); }
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);

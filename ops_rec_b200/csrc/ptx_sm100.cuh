@@ -77,7 +77,6 @@ template <int N> __device__ __forceinline__ void bulk_wait_read() {
 template <int N> __device__ __forceinline__ void bulk_wait() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
-// make this thread's shared-memory writes visible to the async proxy (TMA) before it is asked to read them
 // True in exactly one lane of a converged warp.  Unlike `lane == 0` the compiler sees that a single thread runs the
 // guarded code and keeps its operands in uniform registers.
 __device__ __forceinline__ bool elect_one() {
@@ -93,6 +92,7 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void st_shared_zero16(uint32_t addr) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0u) : "memory");
 }
+// orders this thread's shared-memory accesses before what the async proxy (TMA, tcgen05.mma) is asked to do next
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -256,17 +256,7 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
 //   bits [0,14)  start address >> 4        bits [16,30) leading byte offset >> 4
 //   bits [32,46) stride byte offset >> 4   bits [46,48) descriptor version (1 on sm_100)
 //   bits [61,64) swizzle mode (2 = 128 B)
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-
-// The same descriptor without its start address: OR in (address >> 4); advancing inside a tile adds (bytes >> 4).
+// Here without the start address: OR in (address >> 4); advancing inside a tile adds (bytes >> 4).
 __host__ __device__ constexpr uint64_t umma_desc_sw128_hi(uint32_t lbo_bytes, uint32_t sbo_bytes) {
   return (static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16) | (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32) |
          (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
