@@ -7,11 +7,11 @@
 // tiles of an item only.  Here a CTA is one chain: one 128-row Q tile at a time, K tiles of 64 keys, 192 threads, 128 (D = 64)
 // or 256 (D = 128) columns of tensor memory - so an SM holds four of them (three with a staged bias, two at D = 128), and
 // while one waits the others compute.  64 keys rather than 128: half the columns of tensor memory per chain, and less of a
-// tile lies behind the diagonal or the sequence end.  (4096 sequences of mean 271 with a shared bias, 4 heads of 64: 1192 ->
-// 1149 us; the same histories in a paged cache, 16-80 queries each: 720 -> 540 us
-// with the gather in front of it, 386 us without.  What a step takes - measured inside the
-// kernel, four chains on an SM - is 1 700 cycles of P, SFU-bound, 800 of the two products and their hand-overs, and a
-// tile's start and end add some 8 000.)
+// tile lies behind the diagonal or the sequence end.  (4 heads of 64: 2048 sequences of mean 80 151 ->
+// 103 us, 1024 of mean 300 243 -> 188, but 4096 of mean 271 with a shared bias, three chains on an SM, 1176 -> 1167, no more
+// than the noise; the latter's histories in a paged cache, 16-80 queries each: 720 -> 540 us with a gather in front of it,
+// 386 us without.  What a step takes - measured inside the kernel, four chains on an SM - is 1 700 cycles of P, 800 of the
+// two products and their hand-overs, and a tile's start and end add some 8 000.)
 //
 //   warps 0-3  P / O (thread = row = TMEM lane): scores -> P, output store
 //   warp 4     one thread: draws tiles (scheduler), requests Q, K / V ring and bias tiles by TMA

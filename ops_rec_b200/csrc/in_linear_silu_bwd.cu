@@ -12,8 +12,8 @@
 //   silu_grad_kernel   one read of g and linear_output -> dL [m, n] + per-row-block column sums of dL; HBM-bound
 //   colsum_kernel      the row-block sums -> bias_grad, in a fixed order (bitwise reproducible; no atomics)
 //   launch_product     x_grad = dL . weight and weight_grad = dL^T . x on the forward's tcgen05 pipeline, which reads
-//                      dL, weight and x as they lie.  (Forward + backward of 65536 rows of width 1024: 2448 us with transposed
-//                      copies of all three and one-CTA tiles, 1863 us)
+//                      dL, weight and x as they lie.  (Forward + backward of 65536 rows of width 1024: 2323 us with transposed
+//                      copies of all three and one-CTA tiles, 1760 us)
 // All intermediates live in the caller's workspace.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
