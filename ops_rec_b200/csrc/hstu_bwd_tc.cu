@@ -20,7 +20,7 @@
 // the streamed tile again, read N-major).  TMEM: T1, T2 (128 columns each), Acc1, Acc2 (D columns each).
 // The element-wise stage is split where its inputs are: P and the factor of dS need the scores only and are computed
 // while the dP product runs (dK/dV pass: and dV, and the next step's scores, behind P); dS is then one product per
-// element.  (12 sequences of 4096, 8 heads of 128: dQ pass 663 us, dK/dV pass 836 us; the
+// element.  (12 sequences of 4096, 8 heads of 128: dQ pass 617 us, dK/dV pass 792 us; the
 // element-wise stage - 1 640 + 810 cycles of a dQ step - is what a step takes now.)  The math follows
 // hstu_backward_v1/op_kernel/vector_score.h:159-209 with P and dS rounded to the input type.
 //
